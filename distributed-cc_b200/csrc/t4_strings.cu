@@ -1,5 +1,5 @@
 // The per-block strings of compute_r4_tri (distr_cc/rccsdtq.py:862-1055) in ONE
-// persistent launch over the stored T4 blocks, FP64.
+// persistent launch over the stored T4 blocks, FP64 on the tensor cores.
 //
 // The reference walks its stored blocks (i<=j<=k<=l) and, for each, adds about a
 // hundred strings  r4[q][a,b,c,d] += alpha W[..] . T[..]  whose operands are
@@ -8,12 +8,23 @@
 // are its rows, those in T its columns, the summed letters (one or two of e, f,
 // m, n) its contraction.  Here one CTA owns the output rows a in [a0, a0+na) of
 // one stored block in shared memory and runs every string of a descriptor table
-// over it: each thread takes 4x4 (row, column) micro-tiles of the string's GEMM,
-// reads W and T through strides (operands stay in L2: at nvir ~ 11 the
-// intermediates are a few MB), and adds alpha times its tile into the shared
-// accumulator; one barrier separates consecutive strings, and the block is
-// written once at the end.  The work and memory are those of the stored blocks
-// only, and no operand is gathered or permuted in HBM.
+// over it; the block is written once at the end.
+//
+// Consecutive strings with the same row and column letters (fields 20, 28, 29) form a
+// run: a warp keeps its tile of the run's GEMM in registers (up to 16 8x8 accumulators of
+// mma.m8n8k4.f64) through all of the run's strings and pairs and adds it into the shared
+// accumulator once, so the whole table costs some thirty barriers and shared-memory
+// updates instead of one per string and pair, and a string costs its operand loads and
+// matrix instructions alone.  Operands are read in place through strides (they stay in
+// L1/L2: at nvir ~ 11 the intermediates are a few MB); the plan orders columns and the
+// contraction so that the lanes of a fragment load read neighbouring elements of T or W.
+// A run whose GEMM has one row (the F_oo / W_oooo strings: no output letter in W) is a sum
+// of scaled vectors and runs on the FP64 lanes.
+//
+// What bounds it: operand loads (L1) and the FP64 matrix pipe; the contractions are short
+// (7 to 121 summed values).  Measured (nocc=7, nvir=11, 161 blocks, B200): the kernel 3.5 ms, against
+// 8.3 ms with FP64 lanes, one barrier and one shared-memory update per string and pair; at
+// nocc=5, nvir=8 0.45 against 2.2 ms.
 //
 // The W_ovov / W_voov strings of the OO batch (distr_cc/rccsdtq.py:1062-1349) take a
 // stored SOURCE block and an occupied m per term: they run in "pair mode", once for
@@ -48,16 +59,309 @@ __device__ __forceinline__ int t4s_ostride(int x, int nv) {  // accumulator stri
     return x == 0 ? nv * nv * nv : (x == 1 ? nv * nv : (x == 2 ? nv : 1));
 }
 
+// One string of the table, decoded and checked for this CTA's block (shared memory).
+struct T4Rec {
+    const double *W, *T;  // operands at the block's occupied indices
+    double alpha;
+    int64_t wm, tq;          // pair mode: strides of m (W) and of the source block (T)
+    int64_t wroom, troom;    // elements of W / T past the largest offset the string reaches
+    int rws[4], cts[4];      // strides of the row / column letters by position
+    int K0, wk0, tk0, K1, wk1, tk1;
+    int mask, rord, cord;    // the run key
+    int p0, p1, mode, ok;
+};
+constexpr int T4S_BATCH = 96;  // strings decoded at a time
+
+struct T4Run {  // the GEMM of a run: extents and accumulator strides by position, its tile shape, its end
+    int rext[4], cext[4], ros[4], cos[4];
+    int R, C, shape, end;
+};
+
+// Decode and check descriptor d for block q, rows [a0, a0 + na); returns false when it must
+// not run.
+__device__ bool t4s_decode(const T4StrOps &ops, const int64_t *d, const int *occ, int q, int a0, int na, int nv,
+                           const int32_t *pair_off, int ngroups, int npairs, T4Rec &o, int *status) {
+    const int64_t wop = d[0], top = d[1], mask = d[20], K0 = d[21], wk0 = d[22], tk0 = d[23], K1 = d[24], wk1 = d[25],
+                  tk1 = d[26], rord = d[28], cord = d[29], wm = d[30], mode = d[31];
+    bool ok = wop >= 0 && wop < ops.nops && top >= 0 && top < ops.nops && mask >= 0 && mask < 16 && K0 >= 1 &&
+              K1 >= 1 && wk0 >= 0 && tk0 >= 0 && wk1 >= 0 && tk1 >= 0 && d[10] >= 0 && d[11] >= 0 && rord >= 0 &&
+              rord < 65536 && cord >= 0 && cord < 65536 && wm >= 0 && mode >= 0 && mode <= ngroups;
+    int64_t wb = 0, tb = 0, wmax = 0, tmax = 0;
+    int seen_r = 0, seen_c = 0, npos_r = 0, npos_c = 0;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        const int64_t ws = d[2 + x], ts = d[6 + x], wv = d[12 + x], tv = d[16 + x];
+        const bool inw = (mask >> x) & 1;
+        ok = ok && ws >= 0 && ts >= 0 && wv >= 0 && tv >= 0 && (inw ? tv == 0 : wv == 0);
+        wb += ws * occ[x];
+        tb += ts * occ[x];
+        const int ex = x == 0 ? na : nv;
+        wmax += wv * (ex - 1);
+        tmax += tv * (ex - 1);
+        const int xr = (int)((rord >> (4 * x)) & 15) - 1, xc = (int)((cord >> (4 * x)) & 15) - 1;
+        if (xr >= 0) {
+            npos_r++;
+            seen_r |= 1 << (xr & 7);
+            ok = ok && xr < 4;
+        }
+        if (xc >= 0) {
+            npos_c++;
+            seen_c |= 1 << (xc & 7);
+            ok = ok && xc < 4;
+        }
+        o.rws[x] = (xr >= 0 && xr < 4) ? (int)d[12 + xr] : 0;
+        o.cts[x] = (xc >= 0 && xc < 4) ? (int)d[16 + xc] : 0;
+    }
+    o.mask = (int)mask;
+    o.rord = (int)rord;
+    o.cord = (int)cord;
+    o.mode = (int)mode;
+    o.p0 = 0;
+    o.p1 = 1;
+    // the row order lists the letters of W once each, the column order those of T
+    ok = ok && seen_r == (int)mask && seen_c == (int)(15 & ~mask) && npos_r == __popc(seen_r) &&
+         npos_c == __popc(seen_c);
+    if (ok) {
+        wb += d[10] * q + d[12] * a0;
+        tb += (mode == 0 ? d[11] * q : 0) + d[16] * a0;  // pair mode: field 11 strides the source block
+        wmax += wb + wk0 * (K0 - 1) + wk1 * (K1 - 1);
+        tmax += tb + tk0 * (K0 - 1) + tk1 * (K1 - 1);
+        ok = wmax < ops.n[wop] && tmax < ops.n[top];
+    }
+    if (!ok) {
+        atomicOr(status, 2);
+        return false;
+    }
+    o.W = ops.p[wop] + wb;
+    o.T = ops.p[top] + tb;
+    o.alpha = __longlong_as_double((long long)d[27]);
+    o.wroom = ops.n[wop] - wmax;
+    o.troom = ops.n[top] - tmax;
+    // operands hold fewer than 2^31 elements: a longer pair stride fails for every index but 0
+    o.wm = wm < (1ll << 31) ? wm : (1ll << 31);
+    o.tq = d[11] < (1ll << 31) ? d[11] : (1ll << 31);
+    o.K0 = (int)K0;
+    o.wk0 = (int)wk0;
+    o.tk0 = (int)tk0;
+    o.K1 = (int)K1;
+    o.wk1 = (int)wk1;
+    o.tk1 = (int)tk1;
+    if (mode > 0) {  // once per (source block, m) pair of group mode-1 of this block
+        const int32_t *po = pair_off + (int64_t)q * (ngroups + 1) + (mode - 1);
+        o.p0 = po[0];
+        o.p1 = po[1];
+        if (o.p0 < 0 || o.p1 < o.p0 || o.p1 > npairs) {
+            atomicOr(status, 4);
+            return false;
+        }
+    }
+    return true;
+}
+
+// Operand pointers of pair pr of string r (the string itself when it is not in pair mode);
+// false when the pair fails its checks.
+__device__ __forceinline__ bool t4s_pair(const T4Rec &r, int pr, const int32_t *__restrict__ pair_sm, int nocc,
+                                         const double *&W, const double *&T, int *status) {
+    W = r.W;
+    T = r.T;
+    if (r.mode == 0) return true;
+    const int src = pair_sm[2 * (int64_t)pr], m = pair_sm[2 * (int64_t)pr + 1];
+    if (src < 0 || m < 0 || m >= nocc || r.wm * m >= r.wroom || r.tq * src >= r.troom) {
+        atomicOr(status, 4);
+        return false;
+    }
+    W += r.wm * m;
+    T += r.tq * src;
+    return true;
+}
+
+// The digits of index x in the mixed radix ext, one byte per position (nvir <= 29).
+__device__ __forceinline__ uint32_t t4s_digits(int x, const int *ext) {
+    uint32_t pk = 0;
+#pragma unroll
+    for (int p = 3; p >= 0; --p) {
+        const int y = x / ext[p];
+        pk |= (uint32_t)(x - y * ext[p]) << (8 * p);
+        x = y;
+    }
+    return pk;
+}
+__device__ __forceinline__ int t4s_dot(uint32_t pk, const int *st) {
+    return (int)(pk & 255u) * st[0] + (int)((pk >> 8) & 255u) * st[1] + (int)((pk >> 16) & 255u) * st[2] +
+           (int)(pk >> 24) * st[3];
+}
+
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+// One run on warp tiles of 8 RT rows x 8 CT columns.  Fragments of m8n8k4: lane l holds
+// A[row l/4][k l%4], B[k l%4][col l/4] and D[row l/4][cols 2(l%4), 2(l%4)+1].
+template <int RT, int CT>
+__device__ __forceinline__ void t4s_run(double *acc, const T4Rec *rec, int r0, int r1, const T4Run &g,
+                                        const int32_t *__restrict__ pair_sm, int nocc, int warp, int lane, int *status) {
+    const int nrt = (g.R + 8 * RT - 1) / (8 * RT), nct = (g.C + 8 * CT - 1) / (8 * CT);
+    for (int tile = warp; tile < nrt * nct; tile += T4S_THREADS / 32) {
+        const int rb = (tile / nct) * 8 * RT + (lane >> 2), cb = (tile % nct) * 8 * CT;
+        uint32_t rpk[RT], cpk[CT];
+#pragma unroll
+        for (int u = 0; u < RT; ++u) rpk[u] = t4s_digits(rb + 8 * u < g.R ? rb + 8 * u : 0, g.rext);
+#pragma unroll
+        for (int v = 0; v < CT; ++v) {
+            const int c = cb + 8 * v + (lane >> 2);
+            cpk[v] = t4s_digits(c < g.C ? c : 0, g.cext);
+        }
+        double d[RT][CT][2];
+#pragma unroll
+        for (int u = 0; u < RT; ++u)
+#pragma unroll
+            for (int v = 0; v < CT; ++v) d[u][v][0] = d[u][v][1] = 0.0;
+        for (int s = r0; s < r1; ++s) {
+            const T4Rec &r = rec[s];
+            if (!r.ok) continue;
+            int wo[RT], to[CT];
+#pragma unroll
+            for (int u = 0; u < RT; ++u) wo[u] = t4s_dot(rpk[u], r.rws);
+#pragma unroll
+            for (int v = 0; v < CT; ++v) to[v] = t4s_dot(cpk[v], r.cts);
+            const int K0 = r.K0, K1 = r.K1, wk0 = r.wk0, tk0 = r.tk0, wk1 = r.wk1, tk1 = r.tk1;
+            const int64_t KK = (int64_t)K0 * K1;
+            const double alpha = r.alpha;
+            for (int pr = r.p0; pr < r.p1; ++pr) {
+                const double *W, *T;
+                if (!t4s_pair(r, pr, pair_sm, nocc, W, T, status)) continue;
+                int k0 = lane & 3, k1 = 0;  // this lane's summed values of the step
+                while (k0 >= K0) {
+                    k0 -= K0;
+                    k1++;
+                }
+                for (int64_t kb = 0; kb < KK; kb += 4) {
+                    double a[RT], b[CT];
+                    if (k1 < K1) {
+                        const double *Wk = W + (k0 * wk0 + k1 * wk1), *Tk = T + (k0 * tk0 + k1 * tk1);
+#pragma unroll
+                        for (int u = 0; u < RT; ++u) a[u] = alpha * __ldg(Wk + wo[u]);
+#pragma unroll
+                        for (int v = 0; v < CT; ++v) b[v] = __ldg(Tk + to[v]);
+                    } else {  // past the last summed value
+#pragma unroll
+                        for (int u = 0; u < RT; ++u) a[u] = 0.0;
+#pragma unroll
+                        for (int v = 0; v < CT; ++v) b[v] = 0.0;
+                    }
+                    k0 += 4;
+                    while (k0 >= K0) {
+                        k0 -= K0;
+                        k1++;
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < RT; ++u)
+#pragma unroll
+                        for (int v = 0; v < CT; ++v) dmma(d[u][v][0], d[u][v][1], a[u], b[v]);
+                }
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < CT; ++v)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int c = cb + 8 * v + 2 * (lane & 3) + j;
+                if (c >= g.C) continue;
+                const int oc = t4s_dot(t4s_digits(c, g.cext), g.cos);
+#pragma unroll
+                for (int u = 0; u < RT; ++u)
+                    if (rb + 8 * u < g.R) acc[t4s_dot(rpk[u], g.ros) + oc] += d[u][v][j];
+            }
+    }
+}
+
+// A run whose GEMM has one row: acc[c] += sum of scalar x vector, columns on the lanes.
+__device__ __forceinline__ void t4s_run_vector(double *acc, const T4Rec *rec, int r0, int r1, const T4Run &g,
+                                               const int32_t *__restrict__ pair_sm, int nocc, int *status) {
+    constexpr int V = 8;  // columns of a thread in flight
+    for (int c0 = threadIdx.x; c0 < g.C; c0 += V * T4S_THREADS) {
+        uint32_t cpk[V];
+        double x[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int c = c0 + v * T4S_THREADS;
+            cpk[v] = t4s_digits(c < g.C ? c : 0, g.cext);
+            x[v] = 0.0;
+        }
+        for (int s = r0; s < r1; ++s) {
+            const T4Rec &r = rec[s];
+            if (!r.ok) continue;
+            int to[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) to[v] = t4s_dot(cpk[v], r.cts);
+            for (int pr = r.p0; pr < r.p1; ++pr) {
+                const double *W, *T;
+                if (!t4s_pair(r, pr, pair_sm, nocc, W, T, status)) continue;
+                for (int k1 = 0; k1 < r.K1; ++k1)
+                    for (int k0 = 0; k0 < r.K0; ++k0) {
+                        const double w = r.alpha * __ldg(W + k0 * r.wk0 + k1 * r.wk1);
+                        const double *Tk = T + (k0 * r.tk0 + k1 * r.tk1);
+#pragma unroll
+                        for (int v = 0; v < V; ++v) x[v] = fma(w, __ldg(Tk + to[v]), x[v]);
+                    }
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int c = c0 + v * T4S_THREADS;
+            if (c < g.C) acc[t4s_dot(cpk[v], g.cos)] += x[v];
+        }
+    }
+}
+
+// Issue cost of a run on RT x CT tiles: rounds of the CTA's warps times the matrix
+// instructions and loads of a step.
+__device__ __forceinline__ int t4s_cost(int R, int C, int RT, int CT) {
+    const int n = ((R + 8 * RT - 1) / (8 * RT)) * ((C + 8 * CT - 1) / (8 * CT));
+    return (n + T4S_THREADS / 32 - 1) / (T4S_THREADS / 32) * (2 * RT * CT + RT + CT);
+}
+
+// Tile shapes of a run (8 RT rows x 8 CT columns per warp); -1: one row, on the FP64 lanes.
+__device__ void t4s_plan(T4Run &g, int rord, int cord, int na, int nv) {
+    g.R = g.C = 1;
+    for (int p = 0; p < 4; ++p) {
+        const int xr = ((rord >> (4 * p)) & 15) - 1, xc = ((cord >> (4 * p)) & 15) - 1;
+        g.rext[p] = xr < 0 ? 1 : (xr == 0 ? na : nv);
+        g.ros[p] = xr < 0 ? 0 : t4s_ostride(xr, nv);
+        g.cext[p] = xc < 0 ? 1 : (xc == 0 ? na : nv);
+        g.cos[p] = xc < 0 ? 0 : t4s_ostride(xc, nv);
+        g.R *= g.rext[p];
+        g.C *= g.cext[p];
+    }
+    g.shape = -1;
+    if (g.R == 1) return;
+    const int rt[8] = {4, 4, 3, 2, 8, 1, 8, 2}, ct[8] = {4, 3, 4, 8, 2, 8, 1, 2};
+    int best = 0x7fffffff;
+    for (int i = 0; i < 8; ++i) {  // the shape of least cost for these rows and columns
+        const int c = t4s_cost(g.R, g.C, rt[i], ct[i]);
+        if (c < best) {
+            best = c;
+            g.shape = i;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(T4S_THREADS, 2)
-    k_t4_strings(T4StrOps ops, const int64_t *__restrict__ desc, int nstr, const int32_t *__restrict__ quads,
-                 const int32_t *__restrict__ pair_off, const int32_t *__restrict__ pair_sm, int ngroups, int npairs,
-                 int nocc, int nv, int na_step, int nsplit, double beta, double *__restrict__ r4, int *status) {
+    k_t4_strings(const __grid_constant__ T4StrOps ops, const int64_t *__restrict__ desc, int nstr,
+                 const int32_t *__restrict__ quads, const int32_t *__restrict__ pair_off,
+                 const int32_t *__restrict__ pair_sm, int ngroups, int npairs, int nocc, int nv, int na_step, int nsplit,
+                 double beta, double *__restrict__ r4, int *status) {
     extern __shared__ double acc[];
     const int q = blockIdx.x / nsplit, part = blockIdx.x % nsplit;
     const int a0 = part * na_step;
     const int na = min(na_step, nv - a0);
     const int nv3 = nv * nv * nv;
     const int nacc = na * nv3;
+    T4Rec *rec = reinterpret_cast<T4Rec *>(acc + (int64_t)na_step * nv3);
+    T4Run *runs = reinterpret_cast<T4Run *>(rec + T4S_BATCH);  // runs[i]: the run that starts at rec[i]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int e = threadIdx.x; e < nacc; e += blockDim.x) acc[e] = 0.0;
     int occ[4];
@@ -71,178 +375,58 @@ __global__ void __launch_bounds__(T4S_THREADS, 2)
         if (threadIdx.x == 0) atomicOr(status, 1);
         return;
     }
-    for (int s = 0; s < nstr; ++s) {
-        __syncthreads();  // the previous string's tiles are in acc
-        const int64_t *d = desc + (int64_t)s * T4S_DESC;
-        const int64_t wop = d[0], top = d[1], mask = d[20], K0 = d[21], wk0 = d[22], tk0 = d[23], K1 = d[24],
-                      wk1 = d[25], tk1 = d[26], rord = d[28], cord = d[29], wm = d[30], mode = d[31];
-        const double alpha = __longlong_as_double((long long)d[27]);
-        // ---- checks (uniform: every thread reads the same descriptor)
-        bool ok = wop >= 0 && wop < ops.nops && top >= 0 && top < ops.nops && mask >= 0 && mask < 16 && K0 >= 1 &&
-                  K1 >= 1 && wk0 >= 0 && tk0 >= 0 && wk1 >= 0 && tk1 >= 0 && d[10] >= 0 && d[11] >= 0 &&
-                  rord >= 0 && rord < 65536 && cord >= 0 && cord < 65536 && wm >= 0 && mode >= 0 && mode <= ngroups;
-        int64_t wb = 0, tb = 0, wmax = 0, tmax = 0;
-        int seen_r = 0, seen_c = 0, npos_r = 0, npos_c = 0;
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const int64_t ws = d[2 + x], ts = d[6 + x], wv = d[12 + x], tv = d[16 + x];
-            const bool inw = (mask >> x) & 1;
-            ok = ok && ws >= 0 && ts >= 0 && wv >= 0 && tv >= 0 && (inw ? tv == 0 : wv == 0);
-            wb += ws * occ[x];
-            tb += ts * occ[x];
-            const int ex = x == 0 ? na : nv;
-            wmax += wv * (ex - 1);
-            tmax += tv * (ex - 1);
-            const int xr = (int)((rord >> (4 * x)) & 15) - 1, xc = (int)((cord >> (4 * x)) & 15) - 1;
-            if (xr >= 0) {
-                npos_r++;
-                seen_r |= 1 << (xr & 7);
-                ok = ok && xr < 4;
-            }
-            if (xc >= 0) {
-                npos_c++;
-                seen_c |= 1 << (xc & 7);
-                ok = ok && xc < 4;
-            }
+    for (int s0 = 0, nb; s0 < nstr; s0 += nb) {
+        nb = min(T4S_BATCH, nstr - s0);
+        __syncthreads();  // the previous batch's runs are done with rec
+        if (threadIdx.x < nb) {
+            T4Rec o = {};
+            o.ok = t4s_decode(ops, desc + (int64_t)(s0 + threadIdx.x) * T4S_DESC, occ, q, a0, na, nv, pair_off, ngroups,
+                              npairs, o, status);
+            rec[threadIdx.x] = o;
         }
-        // the row order lists the letters of W once each, the column order those of T
-        ok = ok && seen_r == (int)mask && seen_c == (int)(15 & ~mask) && npos_r == __popc(seen_r) &&
-             npos_c == __popc(seen_c);
-        if (ok) {
-            wb += d[10] * q + d[12] * a0;
-            tb += (mode == 0 ? d[11] * q : 0) + d[16] * a0;  // pair mode: field 11 strides the source block
-            wmax += wb + wk0 * (K0 - 1) + wk1 * (K1 - 1);
-            tmax += tb + tk0 * (K0 - 1) + tk1 * (K1 - 1);
-            ok = wmax < ops.n[wop] && tmax < ops.n[top];
+        __syncthreads();
+        auto same = [&](int i, int j) {
+            return rec[i].mask == rec[j].mask && rec[i].rord == rec[j].rord && rec[i].cord == rec[j].cord;
+        };
+        if (s0 + nb < nstr) {  // a run the batch cuts goes to the next batch whole (unless it fills this one)
+            int e = nb - 1;
+            while (e > 0 && same(e, e - 1)) e--;
+            if (e > 0) nb = e;
         }
-        if (!ok) {
-            if (threadIdx.x == 0) atomicOr(status, 2);
-            continue;
+        if (threadIdx.x < nb && (threadIdx.x == 0 || !same(threadIdx.x, threadIdx.x - 1))) {
+            const int i = threadIdx.x;
+            int e = i;
+            bool any = false;
+            for (; e < nb && same(i, e); e++) any = any || rec[e].ok;
+            if (any) t4s_plan(runs[i], rec[i].rord, rec[i].cord, na, nv);
+            runs[i].end = any ? e : -e;  // no string of the run passed its checks: skipped
         }
-        // ---- the string as a GEMM: rows = W's output letters in the row order (the last
-        // position fastest), columns = T's in the column order
-        int rext[4], cext[4], rws[4], cts[4], ros[4], cos_[4];
-        int R = 1, C = 1;
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const int xr = (int)((rord >> (4 * p)) & 15) - 1, xc = (int)((cord >> (4 * p)) & 15) - 1;
-            rext[p] = xr < 0 ? 1 : (xr == 0 ? na : nv);
-            rws[p] = xr < 0 ? 0 : (int)d[12 + xr];
-            ros[p] = xr < 0 ? 0 : t4s_ostride(xr, nv);
-            cext[p] = xc < 0 ? 1 : (xc == 0 ? na : nv);
-            cts[p] = xc < 0 ? 0 : (int)d[16 + xc];
-            cos_[p] = xc < 0 ? 0 : t4s_ostride(xc, nv);
-            R *= rext[p];
-            C *= cext[p];
-        }
-        const int wk0i = (int)wk0, tk0i = (int)tk0, wk1i = (int)wk1, tk1i = (int)tk1, K0i = (int)K0, K1i = (int)K1;
-        // a warp tile: Lr x Lc lanes, each lane 4 consecutive rows x 4 columns strided by Lc,
-        // so a warp's loads of T cover Lc consecutive columns and its loads of W broadcast
-        const int Lc = C > 64 ? 32 : (C > 32 ? 16 : (C > 16 ? 8 : (C > 8 ? 4 : (C > 4 ? 2 : 1))));
-        const int Lr = 32 / Lc;
-        const int lr = lane / Lc, lc = lane % Lc;
-        const int nrt = (R + 4 * Lr - 1) / (4 * Lr), nct = (C + 4 * Lc - 1) / (4 * Lc);
-        // pair mode: once per (source block, m) pair of group mode-1 of this block
-        int p0 = 0, p1 = 1;
-        if (mode > 0) {
-            const int32_t *po = pair_off + (int64_t)q * (ngroups + 1) + (mode - 1);
-            p0 = po[0];
-            p1 = po[1];
-            if (p0 < 0 || p1 < p0 || p1 > npairs) {
-                if (threadIdx.x == 0) atomicOr(status, 4);
+        __syncthreads();
+        for (int r0 = 0, r1; r0 < nb; r0 = r1) {
+            const T4Run &g = runs[r0];
+            r1 = g.end;
+            if (r1 < 0) {
+                r1 = -r1;
                 continue;
             }
+#define T4S_CASE(ID, RT, CT)                                                             \
+    case ID:                                                                             \
+        t4s_run<RT, CT>(acc, rec, r0, r1, g, pair_sm, nocc, warp, lane, status);          \
+        break;
+            switch (g.shape) {
+                T4S_CASE(0, 4, 4)
+                T4S_CASE(1, 4, 3)
+                T4S_CASE(2, 3, 4)
+                T4S_CASE(3, 2, 8)
+                T4S_CASE(4, 8, 2)
+                T4S_CASE(5, 1, 8)
+                T4S_CASE(6, 8, 1)
+                T4S_CASE(7, 2, 2)
+                default: t4s_run_vector(acc, rec, r0, r1, g, pair_sm, nocc, status);
+            }
+#undef T4S_CASE
+            __syncthreads();  // the next run's tiles split the accumulator another way
         }
-        for (int pr = p0; pr < p1; ++pr) {
-        int64_t wbp = wb, tbp = tb;
-        if (mode > 0) {  // uniform: every thread reads the same pair
-            const int src = pair_sm[2 * (int64_t)pr], m = pair_sm[2 * (int64_t)pr + 1];
-            const int64_t dw = wm * m, dt = d[11] * src;
-            if (src < 0 || m < 0 || m >= nocc || wmax + dw >= ops.n[wop] || tmax + dt >= ops.n[top]) {
-                if (threadIdx.x == 0) atomicOr(status, 4);
-                continue;
-            }
-            wbp += dw;
-            tbp += dt;
-        }
-        const double *W = ops.p[wop] + wbp;
-        const double *T = ops.p[top] + tbp;
-        for (int tile = warp; tile < nrt * nct; tile += T4S_THREADS / 32) {
-            const int r0 = (tile / nct) * 4 * Lr + lr * 4, c0 = (tile % nct) * 4 * Lc + lc;
-            int wo[4], to[4], oR[4], oC[4];
-            bool rv[4], cv[4];
-            int dg[4];  // digits of row r0 (position p), then stepped by one row at a time
-            {
-                int r = r0 < R ? r0 : 0;
-#pragma unroll
-                for (int p = 3; p >= 0; --p) {
-                    dg[p] = r % rext[p];
-                    r /= rext[p];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                rv[u] = r0 + u < R;
-                int o = 0, oa = 0;
-#pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    o += rws[p] * dg[p];
-                    oa += ros[p] * dg[p];
-                }
-                wo[u] = rv[u] ? o : 0;
-                oR[u] = oa;
-                bool carry = true;  // next row
-#pragma unroll
-                for (int p = 3; p >= 0; --p) {
-                    if (carry) {
-                        dg[p] += 1;
-                        carry = dg[p] >= rext[p];
-                        if (carry) dg[p] = 0;
-                    }
-                }
-                int c = c0 + u * Lc;
-                cv[u] = c < C;
-                c = cv[u] ? c : 0;
-                o = 0;
-                oa = 0;
-#pragma unroll
-                for (int p = 3; p >= 0; --p) {
-                    const int ix = c % cext[p];
-                    c /= cext[p];
-                    o += cts[p] * ix;
-                    oa += cos_[p] * ix;
-                }
-                to[u] = o;
-                oC[u] = oa;
-            }
-            double cacc[4][4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) cacc[u][v] = 0.0;
-            for (int k1 = 0; k1 < K1i; ++k1) {
-                const double *Wk = W + k1 * wk1i;
-                const double *Tk = T + k1 * tk1i;
-                for (int k0 = 0; k0 < K0i; ++k0, Wk += wk0i, Tk += tk0i) {
-                    double av[4], bv[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        av[u] = __ldg(Wk + wo[u]);
-                        bv[u] = __ldg(Tk + to[u]);
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) cacc[u][v] = fma(av[u], bv[v], cacc[u][v]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    if (rv[u] && cv[v]) acc[oR[u] + oC[v]] += alpha * cacc[u][v];
-        }
-        }  // pairs: a string's micro-tiles belong to the same threads for every pair
     }
     __syncthreads();
     double *out = r4 + (int64_t)q * nv * nv3 + (int64_t)a0 * nv3;
@@ -262,12 +446,23 @@ extern "C" int dcc_t4_strings_rows_per_cta(int64_t nq, int64_t nvir) {
     const int64_t row = nvir * nvir * nvir * (int64_t)sizeof(double);
     const int64_t na_max = T4S_SMEM_MAX / row;
     if (na_max < 1) return -1;
-    // at least ~3 CTAs per SM over the stored blocks, within the shared-memory limit
-    int64_t nsplit = (3 * 148 + nq - 1) / nq;
-    nsplit = nsplit < 1 ? 1 : (nsplit > nvir ? nvir : nsplit);
-    int64_t na = (nvir + nsplit - 1) / nsplit;
-    if (na > na_max) na = na_max;
-    return (int)na;
+    // Rounds of resident CTAs (two per SM while their accumulators fit) times a CTA's time, which
+    // grows as about 2.5 + na (measured at nocc=7, nvir=11, ms a round: na=1 0.95, 2 1.48, 3 1.70,
+    // 4 1.77, 6 3.0; the best choices 3.6 ms there at na=4 against 5.1 at 3, 0.47 ms at nocc=5,
+    // nvir=8 at na=2 against 0.86 at 1, 0.80 ms at nocc=4, nvir=12 at na=1 against 0.88 at 2).
+    int64_t best_na = 1;
+    double best = 1e300;
+    for (int64_t na = 1; na <= nvir && na <= na_max; na++) {
+        const int64_t smem = na * row + T4S_BATCH * (int64_t)(sizeof(T4Rec) + sizeof(T4Run)) + 1024;
+        const int64_t slots = 148 * (2 * smem <= 228 * 1024 ? 2 : 1);
+        const int64_t rounds = (nq * ((nvir + na - 1) / na) + slots - 1) / slots;
+        const double cost = (double)rounds * (2.5 + (double)na);
+        if (cost < best) {
+            best = cost;
+            best_na = na;
+        }
+    }
+    return (int)best_na;
 }
 
 extern "C" int dcc_t4_strings(const double *const *ops, const int64_t *op_numel, int nops, const int64_t *desc,
@@ -296,9 +491,10 @@ extern "C" int dcc_t4_strings(const double *const *ops, const int64_t *op_numel,
     const int nsplit = (int)((nvir + na - 1) / na);
     const int64_t grid = nq * nsplit;
     DCC_REQUIRE(grid < (1LL << 31), DCC_ERR_SHAPE, "too many blocks");
-    const size_t smem = (size_t)na * nvir * nvir * nvir * sizeof(double);
-    static_assert(T4S_SMEM_MAX <= 227 * 1024, "shared memory per CTA");
-    cudaFuncSetAttribute(k_t4_strings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T4S_SMEM_MAX);
+    const size_t smem = (size_t)na * nvir * nvir * nvir * sizeof(double) + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run));
+    static_assert(T4S_SMEM_MAX + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run)) <= 227 * 1024, "shared memory per CTA");
+    cudaFuncSetAttribute(k_t4_strings, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(T4S_SMEM_MAX + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run))));
     k_t4_strings<<<(unsigned)grid, T4S_THREADS, smem, as_stream(stream)>>>(
         o, desc, nstr, quads, pair_off, pair_sm, ngroups, (int)npairs, (int)nocc, (int)nvir, na, nsplit, beta, r4,
         status);

@@ -201,9 +201,9 @@ def _einsum(kind, subs, X, Y, out, alpha):
         contract.einsum_into(subs, X, Y, out, alpha, 1.0, kind)
 
 
-def build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spin4, T4full=None):
+def build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spin4, T4full=None, T4s=None):
     """The W builders of distr_cc/rccsdtq.py:700-833 as full tensors (FP64, torch).  T4full:
-    unpack_all_orderings(t4) when the caller has it already."""
+    unpack_all_orderings(t4) when the caller has it already; T4s: P4_201 of every block of it."""
     e = torch.einsum
     o, v = slice(0, nocc), slice(nocc, None)
     W = {}
@@ -217,8 +217,9 @@ def build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spi
     X = e('mnek,ijae->kjinma', eris[o, o, v, o], t2) + 0.5 * e('mnef,ijkaef->kjinma', eris[o, o, v, v], t3)
     W["W_ooooov"] = X + X.permute(1, 0, 2, 4, 3, 5)
     # W_oooovv / W_oovvvv: the T4 sums over every ordering (P4_201 applied per ordering)
-    T4s = unpack_all_orderings(t4, nocc) if T4full is None else T4full.clone()
-    spin4(T4s)
+    if T4s is None:
+        T4s = unpack_all_orderings(t4, nocc) if T4full is None else T4full.clone()
+        spin4(T4s)
     Woo = 0.5 * e('mief,ijklfabe->jklmab', eris[o, o, v, v], T4s)
     Word = -0.5 * e('jief,ijklfabc->klabce', eris[o, o, v, v], T4s)
     del T4s
@@ -263,12 +264,35 @@ _FUSED_OPS = ("W_vvvo", "W_vooo", "W_oovvvo", "W_ovovvo", "W_ovovvo_s", "W_ooooo
               "t3", "t3p", "t3s", "t2")
 _DENSE_OPS = ("Wf", "W_vvvv")
 _OO_OPS = ("F_oo", "W_oooo", "T4full", "W_ovov", "W_voov", "T3", "V0", "V1", "V2", "V3")
+_OO_FULL_OPS = ("F_oo", "W_oooo", "T4full", "T4s", "W_ovov", "W_exch")
 # the F_oo / W_oooo prefactor slots of the OO batch as strings over every ordering (subscripts, alpha)
 _OO_PLAIN = (("F_oo", "mi", "mjklabcd", -1.0), ("F_oo", "mj", "imklabcd", -1.0), ("F_oo", "mk", "ijmlabcd", -1.0),
              ("F_oo", "ml", "ijkmabcd", -1.0), ("W_oooo", "mnij", "mnklabcd", 1.0),
              ("W_oooo", "mnik", "mjnlabcd", 1.0), ("W_oooo", "mnil", "mjknabcd", 1.0),
              ("W_oooo", "mnjk", "imnlabcd", 1.0), ("W_oooo", "mnjl", "imknabcd", 1.0),
              ("W_oooo", "mnkl", "ijmnabcd", 1.0))
+
+
+def _oo_full():
+    """The W_ovov / W_voov strings of the OO batch (_OO_TABLE) over every ordering of T4, as
+    (W, W subscripts, T, T subscripts, alpha).  For the output pair (o, v) at position g and with
+    m in place of o, the table's strings over all sources and cases sum to
+        - sum_x sum_me W_ovov[m,x,o,e] T[m..; x -> e]                       (x = a, b, c, d)
+        + sum_me (W_voov[v,m,o,e] + W_ovov[m,v,o,e]) / 2  Ts[m..; v -> e],  Ts = P4_201(T):
+    a V form is Ts with m's axis first, and the three exchanges that accompany W_ovov[m,v,o,e]
+    are 2 T - Ts.  m comes first in T's ordering, so that it takes the earlier axis of a source
+    block in which it occurs twice, as the table's cases do."""
+    out = []
+    for g in range(4):
+        o, v = "ijkl"[g], "abcd"[g]
+        occ = "m" + "ijkl".replace(o, "")
+        rest = v + "abcd".replace(v, "")
+        for x in "abcd":
+            out.append(("W_ovov", "m" + x + o + "e", "T4full", occ + rest.replace(x, "e"), -1.0))
+        out.append(("W_exch", "m" + v + o + "e", "T4s", occ + rest.replace(v, "e"), 1.0))
+    return out
+
+
 _T_OPERAND = {"t3": "t3", "t3_m": "t3", "t3_mn": "t3", "t3p_m": "t3p", "t3s_m": "t3s", "t2_m": "t2", "t2": "t2"}
 
 
@@ -279,7 +303,8 @@ def _operand_shapes(nocc, nv, nq):
             "W_oooovv": (o, o, o, o, v, v), "W_oovvvv": (o, o, v, v, v, v), "t3": (o, o, o, v, v, v),
             "t3p": (o, o, o, v, v, v), "t3s": (o, o, o, v, v, v), "t2": (o, o, v, v), "Wf": (v, v, v, v),
             "W_vvvv": (v, v, v, v), "t4": (nq, v, v, v, v), "F_oo": (o, o), "W_oooo": (o, o, o, o),
-            "T4full": (o, o, o, o, v, v, v, v), "W_ovov": (o, v, o, v), "W_voov": (v, o, o, v),
+            "T4full": (o, o, o, o, v, v, v, v), "T4s": (o, o, o, o, v, v, v, v), "W_exch": (o, v, o, v),
+            "W_ovov": (o, v, o, v), "W_voov": (v, o, o, v),
             "T3": (nq, v, v, v, v), "V0": (nq, v, v, v, v), "V1": (nq, v, v, v, v), "V2": (nq, v, v, v, v),
             "V3": (nq, v, v, v, v)}
 
@@ -322,13 +347,24 @@ def string_descriptor(wsubs, wshape, wop, tsubs, tshape, top, alpha, mode=0):
         else:
             d[16 + n] = ts[tsubs.index(c)]
     d[20] = mask
-    # iteration orders: W's output letters (rows) and T's (columns), slowest first, the
-    # letter with the smallest stride last; nibble p holds letter + 1 of position p
-    rows = sorted((n for n in range(4) if mask >> n & 1), key=lambda n: -d[12 + n])
-    cols = sorted((n for n in range(4) if not mask >> n & 1), key=lambda n: -d[16 + n])
+    # iteration orders: W's output letters (rows) and T's (columns), alphabetical, except that the
+    # columns' letter with T's smallest stride comes last (fastest) unless the summed letters are
+    # the contiguous ones, and the rows' when it is contiguous in W: the eight rows or columns
+    # of a matrix fragment are then neighbours in memory, and strings with the same orders
+    # share a run of the kernel.  Nibble p holds letter + 1 of position p.
+    summed = [c for c in wsubs if c not in "ijklqabcdMQ"]
+
+    def order(letters, strides, unit_only):
+        low = min(letters, key=lambda n: strides[n]) if letters else None
+        if low is None or (unit_only and strides[low] != 1):
+            return sorted(letters)
+        return sorted(n for n in letters if n != low) + [low]
+
+    rows = order([n for n in range(4) if mask >> n & 1], d[12:16], True)
+    cols = order([n for n in range(4) if not mask >> n & 1], d[16:20],
+                 any(c in tsubs and ts[tsubs.index(c)] == 1 for c in summed))
     d[28] = sum((n + 1) << (4 * p) for p, n in enumerate(rows))
     d[29] = sum((n + 1) << (4 * p) for p, n in enumerate(cols))
-    summed = [c for c in wsubs if c not in "ijklqabcdMQ"]
     if sorted(summed) != sorted(c for c in tsubs if c not in "ijklqabcdMQ") or len(summed) > 2:
         raise ValueError("at most two summed letters, each in both operands")
     ks = []
@@ -336,6 +372,7 @@ def string_descriptor(wsubs, wshape, wop, tsubs, tshape, top, alpha, mode=0):
         if wshape[wsubs.index(c)] != tshape[tsubs.index(c)]:
             raise ValueError("extents of %s differ" % c)
         ks.append((wshape[wsubs.index(c)], ws[wsubs.index(c)], ts[tsubs.index(c)]))
+    ks.sort(key=lambda k: min(k[1:]))  # the closest neighbours in memory innermost
     ks += [(1, 0, 0)] * (2 - len(ks))
     d[21:24], d[24:27] = ks[0], ks[1]
     d[27] = struct.unpack("<q", struct.pack("<d", float(alpha)))[0]
@@ -348,13 +385,16 @@ def fused_plan(nocc, nv, dense, device, oo=False):
     strings of dense_vvvv_fvv_ (W_vvvv with F_vv folded into its first and last string); with
     `oo` the OO batch: the F_oo / W_oooo strings over the unpacked T4 of every ordering and
     every W_ovov / W_voov string of _OO_TABLE in pair mode over oo_pairs (pair lists
-    (pair_off [nq, 17], pair_sm [npairs, 2]), None without `oo`)."""
+    (pair_off [nq, 17], pair_sm [npairs, 2]), None without `oo`); oo="full": the W_ovov /
+    W_voov strings over every ordering instead (_oo_full, no pair lists): 20 strings of
+    K = nocc nvir in place of 104 of K = nvir over some 26 pairs a block (nocc=7: 1540 against
+    1830 summed values per element)."""
     def build():
         quads = stored_quadruples(nocc)
         nq = len(quads)
         shp = _operand_shapes(nocc, nv, nq)
         names = list(_FUSED_OPS) + (["t4"] if dense or oo else []) + (list(_DENSE_OPS) if dense else []) + \
-            (list(_OO_OPS) if oo else [])
+            (list(_OO_FULL_OPS if oo == "full" else _OO_OPS) if oo else [])
         rows = []
         for sub, wn, ws, tn, ts, al in _R4_STRINGS:
             sw, st = sub.split(",")
@@ -372,6 +412,10 @@ def fused_plan(nocc, nv, dense, device, oo=False):
             for wn, ws, ts, al in _OO_PLAIN:
                 rows.append(string_descriptor(ws, shp[wn], names.index(wn), ts, shp["T4full"],
                                               names.index("T4full"), al))
+        if oo == "full":
+            for wn, ws, tn, ts, al in _oo_full():
+                rows.append(string_descriptor(ws, shp[wn], names.index(wn), ts, shp[tn], names.index(tn), al))
+        elif oo:
             groups = sorted(oo_pairs(nocc))
             for gid, (g, c) in enumerate(groups):
                 x = "ijkl"[g]
@@ -399,9 +443,14 @@ def fused_plan(nocc, nv, dense, device, oo=False):
                 off.append(row)
             pairs = (torch.tensor(off, dtype=torch.int32, device=device),
                      torch.tensor(sm, dtype=torch.int32, device=device).view(-1, 2))
+        # strings with the same row and column orders side by side (the kernel runs them as one GEMM)
+        first = {}
+        for r in rows:
+            first.setdefault((r[20], r[28], r[29]), len(first))
+        rows.sort(key=lambda r: first[r[20], r[28], r[29]])
         return (torch.tensor(rows, dtype=torch.int64, device=device),
                 torch.tensor(quads, dtype=torch.int32, device=device), names, pairs)
-    return _cached(("fused", nocc, nv, bool(dense), bool(oo)), device, build)
+    return _cached(("fused", nocc, nv, bool(dense), oo), device, build)
 
 
 def fused_status(device):
@@ -444,20 +493,24 @@ def compute_r4_tri_(r4, eris, F_vv, W_vvvo, W_vooo, W_vvvv, W_oooo, W_ovov, t2, 
     if t3.is_cuda and _c_rccsdtq.t4_strings_rows_per_cta(nq, nv) >= 1:
         # every string of every stored block in one launch (FP64), the OO batch included when
         # F_oo is given; the W_vvvv strings join it in FP64 and run as split GEMMs otherwise
-        dense, oo = kind is None, F_oo is not None
+        dense = kind is None
+        oo = False if F_oo is None else ("full" if forms is None else True)
         T4full = unpack_all_orderings(t4, nocc)
-        W = build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spin4, T4full=T4full)
+        T4s = T4full.clone()
+        spin4(T4s)
+        W = build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spin4, T4full=T4full, T4s=T4s)
         W["W_vvvo"], W["W_vooo"] = W_vvvo, W_vooo
         desc, quads, names, pairs = fused_plan(nocc, nv, dense, t3.device, oo=oo)
         ops = dict(W, t3=t3, t3p=t3p, t3s=t3 + t3.permute(0, 1, 2, 4, 5, 3), t2=t2, t4=t4)
         if dense:
             ops.update(Wf=w_with_f(W_vvvv, F_vv), W_vvvv=W_vvvv)
         if oo:
-            if forms is None:
-                forms = lambda t: _c_rccsdtq.t4_forms_batched(t, nv)  # noqa: E731
+            ops.update(F_oo=F_oo, W_oooo=W_oooo, T4full=T4full, T4s=T4s, W_ovov=W_ovov)
+        if oo == "full":
+            ops["W_exch"] = 0.5 * (W_ovvo.permute(0, 1, 3, 2) + W_ovov)
+        elif oo:  # the caller's block forms: the strings of _OO_TABLE over the pair lists
             T3f, V = forms(t4)
-            ops.update(F_oo=F_oo, W_oooo=W_oooo, T4full=T4full, W_ovov=W_ovov,
-                       W_voov=W_ovvo.permute(1, 0, 3, 2), T3=T3f, V0=V[0], V1=V[1], V2=V[2], V3=V[3])
+            ops.update(W_voov=W_ovvo.permute(1, 0, 3, 2), T3=T3f, V0=V[0], V1=V[1], V2=V[2], V3=V[3])
         _c_rccsdtq.t4_strings([ops[n].contiguous() for n in names], desc, quads, nocc, nv, r4.view(nq, -1),
                               0.0, fused_status(t3.device), pairs=pairs)
         if not dense:

@@ -166,6 +166,40 @@ def test_fused_strings_checks():
         assert torch.isfinite(r4).all(), bad
 
 
+@pytest.mark.parametrize("no,nv", [(3, 1), (3, 2), (3, 8), (4, 9), (5, 7), (6, 4), (4, 20)])
+def test_fused_strings_tiles(no, nv):
+    """The tile shapes of the strings kernel (one row or column, fewer than one 8 x 8 tile, whole
+    tiles, one element past them, one and many output rows a CTA): every string of the table
+    run alone, so that no two share a run, against the table run as a whole (1e-13 of the
+    largest element: the same products, at most some 6000 per element, in another order)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from dcc import t4_residual as tr, _c_rccsdtq
+    nq = len(tr.stored_quadruples(no))
+    shp = tr._operand_shapes(no, nv, nq)
+    g = torch.Generator(device="cuda").manual_seed(nv)
+    desc, quads, names, pairs = tr.fused_plan(no, nv, True, "cuda", oo="full")
+    ops = [torch.randn(shp[n], dtype=torch.float64, device="cuda", generator=g) for n in names]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    r4 = torch.empty(nq, nv ** 4, dtype=torch.float64, device="cuda")
+    _c_rccsdtq.t4_strings(ops, desc, quads, no, nv, r4, 0.0, status, pairs=pairs)
+    one = torch.zeros_like(r4)
+    for s in range(desc.shape[0]):
+        _c_rccsdtq.t4_strings(ops, desc[s:s + 1], quads, no, nv, one, 1.0, status, pairs=pairs)
+    want = torch.zeros((nq,) + (nv,) * 4, dtype=torch.float64, device="cuda")
+    for (wn, ws, tn, ts, al) in tr._oo_full():  # the newest strings also as einsums over their operands
+        W, T = ops[names.index(wn)], ops[names.index(tn)]
+        full = torch.einsum(ws + "," + ts + "->ijklabcd", W, T).reshape((no ** 4,) + (nv,) * 4)
+        want.add_(full[tr._stored_rows(no, "cuda")], alpha=al)
+    full_only = torch.zeros_like(r4)
+    pick = [i for i, r in enumerate(desc.tolist()) if names[r[1]] in ("T4full", "T4s") and r[20] != 0]
+    _c_rccsdtq.t4_strings(ops, desc[pick].contiguous(), quads, no, nv, full_only, 0.0, status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    assert float((r4 - one).abs().max()) <= 1e-13 * float(r4.abs().max())
+    assert float((full_only.view_as(want) - want).abs().max()) <= 1e-13 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("precision", ["fp64", "bf16x3"])
 @pytest.mark.parametrize("no,nv", [(4, 5), (7, 11)])
 def test_t4_feedback(oracle, precision, no, nv):

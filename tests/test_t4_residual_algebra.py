@@ -200,3 +200,26 @@ def test_fused_descriptors_emulated(oracle, no, nv, oo):
         pairs = (off, sm)
     got = _emulate_fused(desc.numpy(), q.numpy(), [ops[n].numpy() for n in names], nv, pairs)
     np.testing.assert_allclose(got, want, rtol=1e-12, atol=1e-14 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("no,nv", [(3, 4), (4, 3), (5, 3)])
+def test_oo_strings_over_every_ordering(oracle, no, nv):
+    """fused_plan(oo="full"), the W_ovov / W_voov strings over every ordering of T4, gives the r4
+    of the pair-mode strings, for stored blocks without any symmetry among equal occupied
+    indices (1e-13: sums of at most 4 nocc nvir products in another order)."""
+    d = _inputs(no, nv, 31)
+    rng = np.random.default_rng(no)
+    d["t4"] = rng.standard_normal(d["t4"].shape)
+    d["F_oo"] = rng.standard_normal((no, no))
+    d["W_ovvo"] = rng.standard_normal((no, nv, nv, no))
+    t = {k: torch.from_numpy(np.ascontiguousarray(v)) for k, v in d.items()}
+    spin = _spin(oracle, nv)
+    ops = _fused_ops(t, no, nv, oracle, spin, True)
+    ops["T4s"] = spin("P4_201", 4)(ops["T4full"].clone())
+    ops["W_exch"] = (0.5 * (t["W_ovvo"].permute(0, 1, 3, 2) + t["W_ovov"])).contiguous()
+    r4 = []
+    for oo in (True, "full"):
+        desc, quads, names, pairs = tr.fused_plan(no, nv, False, "cpu", oo=oo)
+        pairs = None if pairs is None else tuple(p.numpy() for p in pairs)
+        r4.append(_emulate_fused(desc.numpy(), quads.numpy(), [ops[n].numpy() for n in names], nv, pairs))
+    assert np.abs(r4[0] - r4[1]).max() <= 1e-13 * np.abs(r4[0]).max()

@@ -53,6 +53,23 @@ def t4_spin_summation_quadruple_sym_(src, B0, B1, B2, B3, nvir):
     return B0, B1, B2, B3
 
 
+def t4_unpack_all(t4, src, rank, nocc, nvir):
+    """(T, Ts): the stored blocks t4 [n, nvir^4] unpacked to every ordering [nocc^4, nvir^4] and
+    P4_201 of each, in one launch.  src / rank: int32 [nocc^4] device tensors, the stored block
+    of every ordering (-1: zeros) and its axes (nibble m: the stored block's axis that axis m of
+    the ordering is)."""
+    t4 = L.as_tensor(t4, f64, "t4")
+    src = L.as_tensor(src, torch.int32, "src")
+    rank = L.as_tensor(rank, torch.int32, "rank")
+    if t4.numel() != t4.shape[0] * nvir ** 4 or src.numel() != nocc ** 4 or rank.numel() != nocc ** 4:
+        raise ValueError("t4 must hold nvir^4 blocks, src and rank nocc^4 entries")
+    T = torch.empty((nocc ** 4,) + (nvir,) * 4, dtype=f64, device=t4.device)
+    Ts = torch.empty_like(T)
+    L.call("dcc_t4_unpack_all", L.ptr(t4), L.ptr(src), L.ptr(rank), L.ptr(T), L.ptr(Ts), nocc ** 4, nvir,
+           L.stream_ptr())
+    return T, Ts
+
+
 def t4_forms_batched(t4, nvir, T3=None, V=None):
     """The transpose-add and the four quadruple-symmetrized forms of every block of t4
     [n, nvir^4] in two launches (the forms the OO batch of compute_r4_tri takes per source

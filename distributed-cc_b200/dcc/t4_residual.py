@@ -107,6 +107,18 @@ def _stored_rows(nocc, device):
         [((i * nocc + j) * nocc + k) * nocc + l for i, j, k, l in stored_quadruples(nocc)], device=device))
 
 
+def _unpack_table(nocc, device):
+    """(stored block, packed axis ranks) of every ordered quadruple, int32 [nocc^4] each, as
+    t4_unpack_all takes them."""
+    def build():
+        src, rank = np.full(nocc ** 4, -1, dtype=np.int32), np.zeros(nocc ** 4, dtype=np.int32)
+        for axes, rows, blocks in _unpack_groups(nocc, "cpu"):
+            src[rows.numpy()] = blocks.numpy()
+            rank[rows.numpy()] = sum(r << (4 * m) for m, r in enumerate(axes))
+        return torch.from_numpy(src).to(device), torch.from_numpy(rank).to(device)
+    return _cached(("unpack_table", nocc), device, build)
+
+
 def unpack_all_orderings(t4, nocc):
     """T[o] for every ordered quadruple o: the stored canonical block with its virtual
     axes permuted (axis p of the ordering is axis rank(p) of the canonical block, stable
@@ -484,7 +496,8 @@ def compute_r4_tri_(r4, eris, F_vv, W_vvvo, W_vooo, W_vvvv, W_oooo, W_ovov, t2, 
     nv = t2.shape[2]
     if spin3 is None:
         spin3 = lambda A: _c_rccsdt.t3_spin_summation_inplace_(A, A.numel() // nv ** 3, nv, "P3_201", 1.0, 0.0)  # noqa: E731
-    if spin4 is None:
+    own_spin4 = spin4 is None
+    if own_spin4:
         spin4 = lambda A: _c_rccsdt_q.t4_spin_summation_inplace_(A, A.numel() // nv ** 4, nv, "P4_201", 1.0, 0.0)  # noqa: E731
     t3 = t3.contiguous()
     t3p = t3.clone()
@@ -495,9 +508,13 @@ def compute_r4_tri_(r4, eris, F_vv, W_vvvo, W_vooo, W_vvvv, W_oooo, W_ovov, t2, 
         # F_oo is given; the W_vvvv strings join it in FP64 and run as split GEMMs otherwise
         dense = kind is None
         oo = False if F_oo is None else ("full" if forms is None else True)
-        T4full = unpack_all_orderings(t4, nocc)
-        T4s = T4full.clone()
-        spin4(T4s)
+        if own_spin4 and nv < 128:
+            T4full, T4s = (x.view((nocc,) * 4 + (nv,) * 4) for x in _c_rccsdtq.t4_unpack_all(
+                t4.contiguous(), *_unpack_table(nocc, t4.device), nocc, nv))
+        else:
+            T4full = unpack_all_orderings(t4, nocc)
+            T4s = T4full.clone()
+            spin4(T4s)
         W = build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spin4, T4full=T4full, T4s=T4s)
         W["W_vvvo"], W["W_vooo"] = W_vvvo, W_vooo
         desc, quads, names, pairs = fused_plan(nocc, nv, dense, t3.device, oo=oo)

@@ -348,6 +348,15 @@ DCC_API int dcc_r4_local_tri_divide_e(double *r4_local, const double *eia, const
 DCC_API int dcc_unpack_t4_ijkl_single(const double *t4_local, double *t4_blk, const int64_t *ijkl_to_local_idx, int64_t i,
                               int64_t j, int64_t k, int64_t l, int64_t nocc, int64_t nvir, void *stream);
 
+/* T[o] = the stored T4 blocks unpacked to the ordering o, Ts[o] = P4_201 of it, for norder
+ * orderings at once: src[o] the stored block (-1: zeros), rank[o] the axis of the stored block
+ * that axis m of the ordering is, in nibble m (DEVICE int32 [norder] each; src[o] below the
+ * number of blocks of t4).  T, Ts DEVICE [norder][nvir^4]; nvir < 128.  Replaces
+ * unpack_t4_ijkl_single_ and t4_single_spin_summation_inplace_ over every ordering
+ * (distr_cc/rccsdtq.py:756-775). */
+DCC_API int dcc_t4_unpack_all(const double *t4, const int32_t *src, const int32_t *rank, double *T, double *Ts,
+                              int64_t norder, int64_t nvir, void *stream);
+
 /* send_data[r] = t4_local[ijkl_to_local_idx[requests[r]]] (DEVICE index
  * arrays).  Replaces fill_local_data_ijkl_ (src/rccsdtq.c:1090-1102). */
 DCC_API int dcc_fill_local_data_ijkl(const double *t4_local, double *send_data, const int32_t *requests,

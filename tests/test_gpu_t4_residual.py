@@ -166,6 +166,24 @@ def test_fused_strings_checks():
         assert torch.isfinite(r4).all(), bad
 
 
+@pytest.mark.parametrize("no,nv", [(3, 1), (2, 5), (4, 10), (3, 11), (3, 12), (3, 13)])
+def test_unpack_all_orderings(no, nv):
+    """t4_unpack_all on either side of the staged blocks' size limit (nvir 11), even and odd
+    extents: T equal to the indexed unpack, Ts to the P4_201 kernel on it (== : the same products
+    and sums; a signed zero may differ)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from dcc import t4_residual as tr, _c_rccsdtq, _c_rccsdt_q
+    g = torch.Generator(device="cuda").manual_seed(nv)
+    t4 = torch.randn((len(tr.stored_quadruples(no)),) + (nv,) * 4, dtype=torch.float64, device="cuda", generator=g)
+    T, Ts = _c_rccsdtq.t4_unpack_all(t4, *tr._unpack_table(no, "cuda"), no, nv)
+    want = tr.unpack_all_orderings(t4, no).view(no ** 4, -1)
+    assert torch.equal(T.view(no ** 4, -1), want)
+    ws = want.clone()
+    _c_rccsdt_q.t4_spin_summation_inplace_(ws, no ** 4, nv, "P4_201", 1.0, 0.0)
+    assert torch.equal(Ts.view(no ** 4, -1), ws)
+
+
 @pytest.mark.parametrize("no,nv", [(3, 1), (3, 2), (3, 8), (4, 9), (5, 7), (6, 4), (4, 20)])
 def test_fused_strings_tiles(no, nv):
     """The tile shapes of the strings kernel (one row or column, fewer than one 8 x 8 tile, whole

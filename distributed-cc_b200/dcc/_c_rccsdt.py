@@ -190,6 +190,21 @@ def t3_divide_update_(t3, r3, eia, ijk, nvir_active=None, write_r3=True, norms=N
     return norms
 
 
+def t3_r1_(r1, t3, oovv, ijk, nocc):
+    """r1 [nocc, nvir] += the T3 part of r1 (distr_cc/rccsdt.py:262-296) from the canonical blocks t3
+    [n, nvir^3] of the triples ijk [n, 3] (int32, device) and oovv = <ij|ab>, one pass over t3."""
+    r1, t3, oovv = (L.as_tensor(x, f64, n) for x, n in ((r1, "r1"), (t3, "t3"), (oovv, "oovv")))
+    ijk = L.as_tensor(ijk, i32, "ijk")
+    n, nvir = t3.shape[0], t3.shape[1]
+    if t3.numel() != n * nvir ** 3 or tuple(ijk.shape) != (n, 3) or r1.numel() != nocc * nvir or \
+            oovv.numel() != (nocc * nvir) ** 2:
+        raise ValueError("t3 must be [n, nvir^3], ijk [n, 3], r1 [nocc, nvir], oovv [nocc, nocc, nvir, nvir]")
+    need = int(L.lib().dcc_t3_r1_workspace_bytes(n, nocc, nvir))
+    ws = torch.empty((need + 7) // 8, dtype=f64, device=t3.device)
+    L.call("dcc_t3_r1", L.ptr(t3), L.ptr(oovv), L.ptr(ijk), n, nocc, nvir, L.ptr(r1), L.ptr(ws), need, L.stream_ptr())
+    return r1
+
+
 def redistribute_ijk_to_abc(t3_ijk, nocc, nvir, out=None):
     """T3[i<=j<=k][abc] -> T3[a<=b<=c][ijk] at one rank
     (distr_cc/distribute_t3.py:1544-1642 with src/rccsdt.c:411-561)."""

@@ -65,6 +65,8 @@ _SIGS = {
     "dcc_fill_local_data_ijk": [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp],
     "dcc_r3_tri_divide_e": [c_vp, c_vp, c_vp, c_i64, c_i64, c_vp],
     "dcc_t3_divide_update": [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_int, c_vp, c_vp, c_size, c_vp],
+    "dcc_t3_r1": [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_size, c_vp],
+    "dcc_t3_r1_workspace_bytes": [c_i64, c_i64, c_i64],
     "dcc_redistribute_ijk_to_abc": [c_vp, c_vp, c_i64, c_i64, c_vp],
     "dcc_fill_t3_from_abc": [c_vp] + [c_i64] * 6 + [c_vp, c_i64, c_vp],
     "dcc_t4_project_1_minus_p4_p31_inplace": [c_vp, c_i64, c_i64, c_dbl, c_dbl, c_vp],
@@ -89,7 +91,7 @@ _SIGS = {
     "dcc_t3_update_workspace_bytes": [c_i64, c_i64],
     "dcc_q_epilogue_workspace_bytes": [c_i64, c_i64],
 }
-_SIZE_FUNCS = {"dcc_t3_update_workspace_bytes", "dcc_q_epilogue_workspace_bytes",
+_SIZE_FUNCS = {"dcc_t3_update_workspace_bytes", "dcc_t3_r1_workspace_bytes", "dcc_q_epilogue_workspace_bytes",
                "dcc_q_group_epilogue_workspace_bytes"}
 
 

@@ -4,15 +4,14 @@ The reference loops over canonical blocks and every distinct ordering of
 each, taking the block (take_t3), symmetrizing it (P3_422 / P3_201) and
 issuing small einsums into r1, r2, W_vooo and W_vvvo.  Here:
 
-* r1 (distr_cc/rccsdt.py:270-293): with V = P3_422 of every canonical block
+* r1 (distr_cc/rccsdt.py:270-293; csrc/t3_feedback.cu): with V = P3_422 of every canonical block
   the paired strings of each case collapse to
       r1[i] += c1 <E[j,k], V[a,b,c]>,  r1[j] += c2 <E[i,k], V[b,a,c]>,
       r1[k] += c3 <E[i,j], V[b,c,a]>       (sums over b, c; E = t1_eris[o,o,v,v])
   with (c1, c2, c3) = (1, 1, 1) for i<j<k, (1, 0, 1/2) for i=j<k,
   (1/2, 1, 0) for i<j=k (the 'cb,acb' partner of a 'bc,abc' string is the same
-  sum); the permutations of V move onto E, so three batched GEMMs over t3 itself
-  give all three (no V pass), scattered to r1 by a one-hot product
-  (deterministic).
+  sum); the permutations of V move onto E, so one pass over t3 itself gives all
+  three (no V pass), added to r1 in a fixed order.
 * r2, W_vooo, W_vvvo (distr_cc/rccsdt.py:300-316, 340-358): the distinct
   orderings of all canonical blocks are all ordered (x,y,z) once, so with X =
   P3_201 applied to every block of the unpacked U (dcc_t3_unpack_all), each
@@ -55,10 +54,14 @@ def r1_add_t3_(r1, t1_eris, t3, ijk, nocc, oovv=None, V=None):
       Ra = y0(4E1 - 2E1^T) + y1(-2E1 + E1^T) + y2(E1 - 2E1^T)
       Rb = y0(-2E2 + E2^T) + y1(4E2 - 2E2^T) + y2(-2E2 + E2^T)
       Rc = y0(E3 - 2E3^T) + y1(-2E3 + E3^T) + y2(4E3 - 2E3^T)
-    (E1 = E[j,k], E2 = E[i,k], E3 = E[i,j]), so three batched GEMMs with three right-hand sides
-    read t3 once each and V is never formed.  V: unused (kept for the callers' signature)."""
+    (E1 = E[j,k], E2 = E[i,k], E3 = E[i,j]) and V is never formed.  On a CUDA device one kernel
+    reads every element of t3 once (dcc_t3_r1, nvir <= 128); elsewhere three batched GEMMs with
+    three right-hand sides read it once each.  V: unused (kept for the callers' signature)."""
     n, nvir = t3.shape[0], t3.shape[1]
     E = oovv if oovv is not None else eris_slices(t1_eris, None, nocc)["oovv"]
+    if t3.is_cuda and nvir <= 128 and ijk.dtype == torch.int32 and all(
+            x.dtype == f64 and x.is_contiguous() for x in (r1, t3)) and ijk.is_contiguous() and E.dtype == f64:
+        return _c_rccsdt.t3_r1_(r1, t3, E.contiguous(), ijk, nocc)
     il, jl, kl = ijk[:, 0].long(), ijk[:, 1].long(), ijk[:, 2].long()
     c1, c2, c3 = _case_coefficients(ijk)
     E1, E2, E3 = E[jl, kl], E[il, kl], E[il, jl]  # [n][nvir][nvir]

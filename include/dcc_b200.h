@@ -182,6 +182,14 @@ DCC_API int dcc_t3_divide_update_noalloc(double *t3, double *r3, const double *e
                                          int64_t nblocks, int64_t nvir, int64_t nvir_active, int write_r3,
                                          double *norms, void *stream);
 
+/* r1[nocc][nvir] += the T3 part of r1 (distr_cc/rccsdt.py:262-296) from the canonical blocks t3
+ * [nblocks][nvir^3] of the triples ijk (DEVICE int32 [nblocks][3]) and oovv = <ij|ab>
+ * [nocc][nocc][nvir][nvir], in one pass over t3; a block whose triple lies outside [0, nocc) adds
+ * nothing.  nvir <= 128; workspace of dcc_t3_r1_workspace_bytes bytes (DEVICE). */
+DCC_API size_t dcc_t3_r1_workspace_bytes(int64_t nblocks, int64_t nocc, int64_t nvir);
+DCC_API int dcc_t3_r1(const double *t3, const double *oovv, const int32_t *ijk, int64_t nblocks, int64_t nocc,
+                      int64_t nvir, double *r1, void *workspace, size_t workspace_bytes, void *stream);
+
 /* IJK -> ABC layout transform at one rank: t3_abc[g][x][y][z] (g the rank of
  * a<=b<=c) from t3_ijk[q][a][b][c] (q the rank of i<=j<=k).  Reproduces the
  * record pack + Alltoallv + unpack of distr_cc/distribute_t3.py:1544-1642 with

@@ -58,3 +58,20 @@ def test_intermediates(mods, oracle, no, nv):
     fb.intermediates_t3_add_(dWo, dWv, dev(g), X, no)
     np.testing.assert_allclose(dWo.cpu().numpy(), w1, rtol=0, atol=1e-11 * np.abs(w1).max())
     np.testing.assert_allclose(dWv.cpu().numpy(), w2, rtol=0, atol=1e-11 * np.abs(w2).max())
+
+
+@pytest.mark.parametrize("no,nv", [(1, 3), (2, 1), (3, 31), (3, 32), (2, 33), (2, 65), (2, 96), (2, 97), (1, 128)])
+def test_r1_kernel(mods, no, nv):
+    """The one-pass r1 kernel at the edges of its z tiles (32, 64, 96, 128) and of its groups of four
+    first indices, against the batched GEMMs of the same sums on the CPU (1e-12 of the largest
+    entry: sums of 9 nvir^2 products per block in another order)."""
+    fb, _ = mods
+    g = torch.Generator().manual_seed(nv)
+    ijk = torch.tensor([(i, j, k) for i in range(no) for j in range(i, no) for k in range(j, no)], dtype=torch.int32)
+    t3 = torch.randn(ijk.shape[0], nv, nv, nv, dtype=torch.float64, generator=g)
+    E = torch.randn(no, no, nv, nv, dtype=torch.float64, generator=g)
+    r1 = torch.randn(no, nv, dtype=torch.float64, generator=g)
+    want = fb.r1_add_t3_(r1.clone(), None, t3, ijk, no, oovv=E)
+    got = fb.r1_add_t3_(r1.cuda(), None, t3.cuda(), ijk.cuda(), no, oovv=E.cuda())
+    scale = max(float((want - r1).abs().max()), float(r1.abs().max()))
+    assert float((got.cpu() - want).abs().max()) <= 1e-12 * scale

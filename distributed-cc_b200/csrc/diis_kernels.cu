@@ -159,13 +159,22 @@ __global__ void __launch_bounds__(DI_THREADS) k_diis_combine(DiisPtrs xs, double
     block_sums(none, dd, 0, partial, DI_MAXS + 1);
 }
 
-// out[s] = sum over CTAs of partial[cta][s], CTAs in order.
-__global__ void k_diis_finish(const double *partial, int nblk, int nsum, double *out) {
-    const int s = threadIdx.x;
-    if (s >= nsum) return;
+// out[s] = sum over CTAs of partial[cta][s] (one block per s): each thread a strided subset in
+// order, then a fixed tree.  A single thread per s, adding every CTA's value in turn, took 71 us at
+// 1184 CTAs (a chain of dependent loads); this form 4 us.
+constexpr int DI_FIN = 256;
+__global__ void __launch_bounds__(DI_FIN) k_diis_finish(const double *partial, int nblk, double *out) {
+    __shared__ double red[DI_FIN / 32];
+    const int s = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double x = 0.0;
-    for (int b = 0; b < nblk; b++) x += partial[(int64_t)b * (DI_MAXS + 1) + s];
-    out[s] = x;
+    for (int b = threadIdx.x; b < nblk; b += DI_FIN) x += partial[(int64_t)b * (DI_MAXS + 1) + s];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) red[w] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < DI_FIN / 32; q++) x += red[q];
+        out[s] = x;
+    }
 }
 
 static int make_segs(DiisSegs &g, double *const *seg, const int64_t *seg_n, const double *scale, int nseg,
@@ -259,7 +268,7 @@ extern "C" int dcc_diis_push(double *const *seg, const int64_t *seg_n, const dou
     cudaStream_t st = as_stream(stream);
     double *partial = (double *)workspace;
     k_diis_push<<<DI_GRID, DI_THREADS, 0, st>>>(g, xprev, x_slot, e_slot, eo, partial);
-    k_diis_finish<<<1, 32, 0, st>>>(partial, DI_GRID, nother + 1, dots);
+    k_diis_finish<<<nother + 1, DI_FIN, 0, st>>>(partial, DI_GRID, dots);
     return launch_status("diis_push");
 }
 
@@ -287,6 +296,6 @@ extern "C" int dcc_diis_combine(const double *const *xs, const double *coef, int
     cudaStream_t st = as_stream(stream);
     double *partial = (double *)workspace;
     k_diis_combine<<<DI_GRID, DI_THREADS, 0, st>>>(p, xprev, g, partial);
-    k_diis_finish<<<1, 32, 0, st>>>(partial, DI_GRID, 1, delta);
+    k_diis_finish<<<1, DI_FIN, 0, st>>>(partial, DI_GRID, delta);
     return launch_status("diis_combine");
 }

@@ -20,10 +20,11 @@ issuing small einsums into r1, r2, W_vooo and W_vvvo.  Here:
 All in FP64 (bandwidth-bound: K = nvir or nocc*nvir against 1-6 GB of T3)."""
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from . import _c_rccsdt
-from .t3_residual import unpack_all_
+from .t3_residual import full_dtype, unpack_all_
 
 f64 = torch.float64
 
@@ -179,7 +180,10 @@ class SplitFeedback:
     the split operands (starting on a k-block) and its own GEMM: the tensor cores accumulate in
     FP32 over the other two indices only, and the epilogue sums the nocc partial results in FP64
     -- one FP32 accumulation over the whole contraction (nocc nvir^2 terms at nvir ~ 90) lost
-    four digits to cancellation.  The partial results accumulate in an FP64 scratch T[row][column]
+    four digits to cancellation.  All pieces of both operands are split in one grouped launch and all
+    x problems of a group run as one grouped GEMM (reductions in L2 into the scratch): a problem alone has
+    36 tiles for 148 SMs at nocc=10 / nvir=90 (K = nvir^2), all ten 360.  The partial results
+    accumulate in an FP64 scratch T[row][column]
     (contiguous, so the epilogue writes whole rows; W_vvvo's own layout puts every element of an
     epilogue row in its own sector), and each string's rows are added to its output once, with a
     permutation.  One split buffer of X (nocc^2 nvir x nocc nvir^2 elements, two 2-byte pieces
@@ -238,19 +242,54 @@ class SplitFeedback:
         self._elo = torch.empty(emax, dtype=dt, device=device)
         self._scratch = torch.empty(tmax, dtype=f64, device=device)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self._groups = {}
+        if torch.device(device).type == "cuda":  # run()'s default, so that it uploads no table
+            for group in (("vovv", "wvooo"), ("ooov", "wvvvo")):
+                self._group(group, full_dtype(precision, nvir))
 
     def _operand(self, rows, ks, Kp, hi, lo):
         n = rows * Kp
         buf = (hi[:n].view(rows, Kp), lo[:n].view(rows, Kp))
         return self.c.Split(rows, kind=self.kind, buffers=buf, pieces=ks, align=self.blk)
 
+    def _group(self, group, xdtype):
+        """The grouped split and GEMM of the strings `group` (same columns and contraction) for
+        X of type xdtype: (grouped split, grouped GEMM, E element stride per x, rows M, columns N).
+        Their tables hold addresses of this object's buffers only; X and E are given per run."""
+        key = (tuple(group), xdtype)
+        if key not in self._groups:
+            c, tm = self.c, self.terms[group[0]]
+            pieces, ks, Kp = self.plans[group[0]]
+            R1, R2, S1, S2 = tm["kin"]
+            N, M = tm["N"], sum(self.terms[n]["M"] for n in group)
+            B = self._operand(N, ks, Kp, self._xhi, self._xlo)
+            A = self._operand(M, ks, Kp, self._ehi, self._elo)
+            T = self._scratch[:M * N]
+            es = A.hi.element_size()
+            split, gemm = [], []
+            f32 = 1 if xdtype == torch.float32 else 0
+            for (op, fm, fk, sf) in ((B, tm["fn"], c.three(R1, R2, self.Sx, S1, S2), f32),
+                                     (A, c.lin(self.no * R1 * R2), c.lin(1), 0)):
+                for off, k, w in op.pieces:
+                    split.append([op.hi.data_ptr(), op.lo.data_ptr(), op.M, k, w, op.Kp, off] + list(c.as4(fm))
+                                 + list(c.as4(fk)) + [sf])
+            for off, _, w in A.pieces:
+                gemm.append([A.hi.data_ptr() + off * es, A.lo.data_ptr() + off * es, A.Kp, B.hi.data_ptr() + off * es,
+                             B.lo.data_ptr() + off * es, B.Kp, M, N, w, T.data_ptr(), 0] + list(c.as4(c.lin(N)))
+                            + list(c.as4(c.lin(1))))
+            self._groups[key] = (c.GroupedSplit(split, self.kind, self.dev),
+                                 c.GroupedGemm(gemm, np.ones(len(gemm)), self.kind, self.dev), R1 * R2, M, N)
+        return self._groups[key]
+
     def run(self, X, E, outs, names=("vovv", "ooov", "wvooo", "wvvvo")):
-        """outs[...] += the strings above.  X: [no,no,no,nv,nv,nv] FP64, contiguous; E: the
+        """outs[...] += the strings above.  X: [no,no,no,nv,nv,nv] FP64 or FP32, contiguous; E: the
         slices {'vovv', 'ooov', 'oovv'} of eris_slices on the device; outs: {'r2', 'W_vooo',
         'W_vvvo'} FP64 device tensors.  Strings that read X the same way share one split of X
-        and one GEMM per piece."""
-        c = self.c
-        Xf = X.reshape(-1)
+        and one grouped GEMM."""
+        no, nv = self.no, self.nv
+        if not X.is_cuda or X.dtype not in (f64, torch.float32) or not X.is_contiguous() or \
+                X.numel() != no ** 3 * nv ** 3:
+            raise ValueError("X must be a contiguous FP64 or FP32 [nocc^3, nvir^3] CUDA tensor")
         done = set()
         for name in names:
             if name in done:
@@ -258,22 +297,16 @@ class SplitFeedback:
             tm = self.terms[name]
             group = [n for n in names if n not in done and self.terms[n]["fn"] == tm["fn"]
                      and self.terms[n]["kin"] == tm["kin"] and self.terms[n]["N"] == tm["N"]]
-            pieces, ks, Kp = self.plans[name]
-            R1, R2, S1, S2 = tm["kin"]
-            N = tm["N"]
-            B = self._operand(N, ks, Kp, self._xhi, self._xlo)
-            for i, (x0, xc) in enumerate(pieces):
-                B.fill_piece(i, Xf[x0 * self.Sx:], tm["fn"], c.three(R1, R2, self.Sx, S1, S2))
+            split, gemm, estep, M, N = self._group(group, X.dtype)
             # the strings' E slices stacked: [row][x][k1][k2]
             Ep = torch.cat([E[self.terms[n]["src"]].permute(*self.terms[n]["perm"]) for n in group]).contiguous()
-            M = Ep.shape[0]
-            A = self._operand(M, ks, Kp, self._ehi, self._elo)
-            row = self.no * R1 * R2
-            for i, (x0, xc) in enumerate(pieces):
-                A.fill_piece(i, Ep[:, x0:], c.lin(row), c.lin(1))
+            if Ep.dtype != f64 or not Ep.is_cuda or Ep.numel() != M * no * estep:
+                raise ValueError("the E slices must be FP64 CUDA tensors of nocc / nvir extents")
+            xs, es = self.Sx * X.element_size(), estep * Ep.element_size()
+            split.run([X.data_ptr() + x * xs for x in range(no)] + [Ep.data_ptr() + x * es for x in range(no)])
             T = self._scratch[:M * N].view(M, N)
-            for i, (off, _, w) in enumerate(A.pieces):
-                c.gemm_range_(A, B, T, c.lin(N), c.lin(1), 1.0, 0.0 if i == 0 else 1.0, self.status, off, w)
+            T.zero_()
+            gemm.run(self.status)
             r0 = 0
             for n in group:
                 tn = self.terms[n]

@@ -281,15 +281,37 @@ class SplitFeedback:
                                  c.GroupedGemm(gemm, np.ones(len(gemm)), self.kind, self.dev), R1 * R2, M, N)
         return self._groups[key]
 
+    def _contract(self, group, X, Ep, T):
+        """T = the products of the group's stacked E slices Ep with X, all x in two launches."""
+        split, gemm, estep, M, N = self._group(group, X.dtype)
+        if Ep.dtype != f64 or not Ep.is_cuda or Ep.numel() != M * self.no * estep:
+            raise ValueError("the E slices must be FP64 CUDA tensors of nocc / nvir extents")
+        xs, es = self.Sx * X.element_size(), estep * Ep.element_size()
+        split.run([X.data_ptr() + x * xs for x in range(self.no)] + [Ep.data_ptr() + x * es for x in range(self.no)])
+        T.zero_()
+        gemm.run(self.status)
+
+    def _contract_pieces(self, group, X, Ep, T):
+        c, tm = self.c, self.terms[group[0]]
+        _, ks, Kp = self.plans[group[0]]
+        R1, R2, S1, S2 = tm["kin"]
+        B = self._operand(tm["N"], ks, Kp, self._xhi, self._xlo)
+        A = self._operand(Ep.shape[0], ks, Kp, self._ehi, self._elo)
+        Xf = X.reshape(-1)
+        for x, (off, _, w) in enumerate(A.pieces):
+            B.fill_piece(x, Xf[x * self.Sx:], tm["fn"], c.three(R1, R2, self.Sx, S1, S2))
+            A.fill_piece(x, Ep[:, x:], c.lin(self.no * R1 * R2), c.lin(1))
+            c.gemm_range_(A, B, T, c.lin(tm["N"]), c.lin(1), 1.0, 0.0 if x == 0 else 1.0, self.status, off, w)
+
     def run(self, X, E, outs, names=("vovv", "ooov", "wvooo", "wvvvo")):
         """outs[...] += the strings above.  X: [no,no,no,nv,nv,nv] FP64 or FP32, contiguous; E: the
         slices {'vovv', 'ooov', 'oovv'} of eris_slices on the device; outs: {'r2', 'W_vooo',
         'W_vvvo'} FP64 device tensors.  Strings that read X the same way share one split of X
         and one grouped GEMM."""
         no, nv = self.no, self.nv
-        if not X.is_cuda or X.dtype not in (f64, torch.float32) or not X.is_contiguous() or \
-                X.numel() != no ** 3 * nv ** 3:
-            raise ValueError("X must be a contiguous FP64 or FP32 [nocc^3, nvir^3] CUDA tensor")
+        if X.dtype not in (f64, torch.float32) or X.numel() < no ** 3 * nv ** 3:
+            raise ValueError("X must be an FP64 or FP32 [nocc^3, nvir^3] tensor")
+        X = X.contiguous()
         done = set()
         for name in names:
             if name in done:
@@ -297,16 +319,14 @@ class SplitFeedback:
             tm = self.terms[name]
             group = [n for n in names if n not in done and self.terms[n]["fn"] == tm["fn"]
                      and self.terms[n]["kin"] == tm["kin"] and self.terms[n]["N"] == tm["N"]]
-            split, gemm, estep, M, N = self._group(group, X.dtype)
             # the strings' E slices stacked: [row][x][k1][k2]
             Ep = torch.cat([E[self.terms[n]["src"]].permute(*self.terms[n]["perm"]) for n in group]).contiguous()
-            if Ep.dtype != f64 or not Ep.is_cuda or Ep.numel() != M * no * estep:
-                raise ValueError("the E slices must be FP64 CUDA tensors of nocc / nvir extents")
-            xs, es = self.Sx * X.element_size(), estep * Ep.element_size()
-            split.run([X.data_ptr() + x * xs for x in range(no)] + [Ep.data_ptr() + x * es for x in range(no)])
+            M, N = Ep.shape[0], tm["N"]
             T = self._scratch[:M * N].view(M, N)
-            T.zero_()
-            gemm.run(self.status)
+            if X.is_cuda:
+                self._contract(group, X, Ep, T)
+            else:  # the same pieces one by one (the emulated maps of the CPU tests)
+                self._contract_pieces(group, X, Ep, T)
             r0 = 0
             for n in group:
                 tn = self.terms[n]

@@ -118,17 +118,21 @@ def vjp(lam, t2, t3, F_vv, F_oo, W_vvvo, W_vooo, W_vvvv, W_ovov, W_ovvo, Ws, pre
     gWovvo = E('ijkabc,jklbcd->ladi', Lam, U, z(*W_ovvo.shape), 0.5, 0.0)
     gWovov.add_(gG2, alpha=-0.5)
     gWovvo.add_(gG2.permute(0, 1, 3, 2), alpha=-0.5)
-    # (Ws.U - F_oo.U) / 2
+    # (Ws.U - F_oo.U) / 2.  F_oo's contraction with Lam is the one of Ws at m = j, traced
     gWs = E('ijkabc,lmkabc->lmij', Lam, U, z(*Ws.shape), 0.5, 0.0)
     gWoooo = 0.5 * (gWs + gWs.permute(1, 0, 3, 2))
-    gFoo = E('ijkabc,ljkabc->li', Lam, U, z(*F_oo.shape), -0.5, 0.0)
+    if kind is None or nocc * nvir ** 3 > MAX_SPLIT_K:
+        gFoo = -torch.einsum('ljij->li', gWs)
+    else:  # gWs came from a split product: F_oo's longer contraction keeps its own, in FP64 as ever
+        gFoo = E('ijkabc,ljkabc->li', Lam, U, z(*F_oo.shape), -0.5, 0.0)
     del U
     gU = torch.empty(full, dtype=f64, device=dev)
     E('ijkabc,lbid->jkldca', Lam, W_ovov, gU, -1.0, 0.0)
     E('ijkabc,laid->jkldcb', Lam, G2, gU)
     E('ijkabc,ladi->jklbcd', Lam, W_ovvo, gU, 0.5)
-    E('ijkabc,lmij->lmkabc', Lam, Ws, gU, 0.5)
-    E('ijkabc,li->ljkabc', Lam, F_oo, gU, -0.5)
+    # Ws and F_oo together: F_oo[l,i] at m = j (its own GEMM had nocc columns of a 256-column tile)
+    eye = torch.eye(nocc, dtype=f64, device=dev)
+    E('ijkabc,lmij->lmkabc', Lam, (Ws - F_oo[:, None, :, None] * eye[None, :, None, :]).contiguous(), gU, 0.5)
     del Lam
     # unpack^T then the projection: (1/|stab|) * sum over all six permutations
     gt3 = torch.empty_like(t3)
@@ -144,13 +148,17 @@ def vjp(lam, t2, t3, F_vv, F_oo, W_vvvo, W_vooo, W_vvvv, W_ovov, W_ovvo, Ws, pre
     gFvv = E('qabc,qdbc->ad', lam, t3, z(*F_vv.shape), 1.0, 0.0)
     E('qabc,qadc->bd', lam, t3, gFvv)
     E('qabc,qabd->cd', lam, t3, gFvv)
-    gd = z(*t3.shape)
-    E('qabc,abde->qdec', lam, W_vvvv, gd)
+    gd = torch.empty_like(t3)
+    # F_vv rides in the W operands, as in the forward (contract.WvvvvT3)
+    W1 = W_vvvv.clone()
+    W1.diagonal(0, 1, 3).add_(F_vv.unsqueeze(2))  # F[a,d] delta(b,e)
+    W1.diagonal(0, 0, 2).add_(F_vv.unsqueeze(2))  # delta(a,d) F[b,e]
+    E('qabc,abde->qdec', lam, W1, gd, 1.0, 0.0)
     E('qabc,acde->qdbe', lam, W_vvvv, gd)
-    E('qabc,bcde->qade', lam, W_vvvv, gd)
-    E('qabc,ad->qdbc', lam, F_vv, gd)
-    E('qabc,bd->qadc', lam, F_vv, gd)
-    E('qabc,cd->qabd', lam, F_vv, gd)
+    W1.copy_(W_vvvv)
+    W1.diagonal(0, 0, 2).add_(F_vv.unsqueeze(2))  # delta(b,d) F[c,e]
+    E('qabc,bcde->qade', lam, W1, gd)
+    del W1
     gt3.add_(stab_project(gd, ijk))
     return gt2, gt3, gFvv, gFoo, gWvvvo, gWvooo, gWvvvv, gWovov, gWovvo, gWoooo
 

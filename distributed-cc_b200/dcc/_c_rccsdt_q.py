@@ -5,6 +5,8 @@ e_abcdijkl_division_, t4_spin_summation_inplace_(P4_444),
 t4_multiply_factor_ and the two dot products (distr_cc/rccsdt_q.py:1131-1154)."""
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib as L
@@ -32,6 +34,23 @@ def fill_t3_from_abc(t3_blk_target, a0, a1, b0, b1, nvir, nocc, t3_abc, ld_b):
     L.call("dcc_fill_t3_from_abc", L.ptr(t3_blk_target), a0, a1, b0, b1, nvir, nocc, L.ptr(t3_abc), ld_b,
            L.stream_ptr())
     return t3_blk_target
+
+
+def fill_t3_slabs(targets, ranges, nvir, nocc, t3_abc):
+    """targets[p] = T[a0:a1, b0:b1, :, i, j, k] for up to six ranges (a0, a1, b0, b1), one launch
+    (fill_t3_from_abc of each)."""
+    t3_abc = L.as_tensor(t3_abc, f64, "t3_abc")
+    if t3_abc.numel() != nvir * (nvir + 1) * (nvir + 2) // 6 * nocc ** 3:
+        raise ValueError("t3_abc must hold nvir(nvir+1)(nvir+2)/6 blocks of nocc^3")
+    for t, (a0, a1, b0, b1) in zip(targets, ranges):
+        L.as_tensor(t, f64, "target")
+        if t.numel() < (a1 - a0) * (b1 - b0) * nvir * nocc ** 3:
+            raise ValueError("target too small")
+    n = len(targets)
+    ptrs = (ctypes.c_void_p * n)(*[t.data_ptr() for t in targets])
+    rg = (ctypes.c_int64 * (4 * n))(*[int(x) for r in ranges for x in r])
+    L.call("dcc_fill_t3_slabs", ptrs, rg, n, nvir, nocc, L.ptr(t3_abc), L.stream_ptr())
+    return targets
 
 
 def e_abcdijkl_division_(r4, e_occ, e_vir, a0, a1, b0, b1, c0, c1, d0, d1, blk_a, blk_b, blk_c, blk_d, nocc):

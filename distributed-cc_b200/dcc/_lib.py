@@ -68,6 +68,7 @@ _SIGS = {
     "dcc_t3_r1": [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_size, c_vp],
     "dcc_t3_r1_workspace_bytes": [c_i64, c_i64, c_i64],
     "dcc_redistribute_ijk_to_abc": [c_vp, c_vp, c_i64, c_i64, c_vp],
+    "dcc_fill_t3_slabs": [c_vp, c_vp, c_int, c_i64, c_i64, c_vp, c_vp],
     "dcc_fill_t3_from_abc": [c_vp] + [c_i64] * 6 + [c_vp, c_i64, c_vp],
     "dcc_t4_project_1_minus_p4_p31_inplace": [c_vp, c_i64, c_i64, c_dbl, c_dbl, c_vp],
     "dcc_t4_spin_summation_inplace": [c_vp, c_i64, c_i64, c_str, c_dbl, c_dbl, c_vp],

@@ -391,15 +391,14 @@ class GroupedSplit:
         L.check(_split_grouped_table(spec.ctypes.data_as(L.c_vp), self.n, L.ptr(self.table), nbytes,
                                      ctypes.byref(total)))
         self.total = total.value
-        self._srcs = (L.c_vp * self.n)()
 
     def run(self, srcs):
-        """srcs: n device addresses (ints), operand p read from srcs[p]."""
+        """srcs: n device addresses (ints or an int64 array), operand p read from srcs[p]."""
         if len(srcs) != self.n:
             raise ValueError("need %d sources" % self.n)
-        for i, p in enumerate(srcs):
-            self._srcs[i] = int(p)
-        L.check(_split_grouped(L.ptr(self.table), self.n, self.total, self._srcs, self.kind, L.stream_ptr()))
+        srcs = np.ascontiguousarray(srcs, dtype=np.int64)
+        L.check(_split_grouped(L.ptr(self.table), self.n, self.total, srcs.ctypes.data_as(L.c_vp), self.kind,
+                               L.stream_ptr()))
 
 
 class GroupedGemm:

@@ -361,15 +361,17 @@ class QEnergy:
 
     # ------------------------------------------------------------------ group data
     def _slabs(self, t3_abc, r, which=_SLABS, out=None):
-        """T3 slabs of the group / d-chunk r (FP64, filled on the device)."""
+        """T3 slabs of the group / d-chunk r (FP64, filled on the device by one launch)."""
         nv, no = self.nv, self.no
         rng = {"a": (r[0], r[1]), "b": (r[2], r[3]), "c": (r[4], r[5]), "d": (r[6], r[7])}
         out = {} if out is None else out
-        for s in which:
-            (x0, x1), (y0, y1) = rng[s[1]], rng[s[2]]
-            t = torch.empty((x1 - x0, y1 - y0, nv, no, no, no), dtype=f64, device=self.dev)
-            _c_rccsdt_q.fill_t3_from_abc(t, x0, x1, y0, y1, nv, no, t3_abc, y1 - y0)
-            out[s] = t
+        ranges = [rng[s[1]] + rng[s[2]] for s in which]
+        shapes = [(x1 - x0, y1 - y0, nv, no, no, no) for x0, x1, y0, y1 in ranges]
+        sizes = [sh[0] * sh[1] * nv * no ** 3 for sh in shapes]
+        parts = torch.empty(sum(sizes), dtype=f64, device=self.dev).split(sizes)
+        for s, sh, t in zip(which, shapes, parts):
+            out[s] = t.view(sh)
+        _c_rccsdt_q.fill_t3_slabs(parts, ranges, nv, no, t3_abc)
         return out
 
     def _chunks(self, d0, d1=None):
@@ -495,11 +497,14 @@ class QEnergy:
             P["alpha"].append(pr["alpha"])
         plan = {"zero": self._pool.narrow(0, 0, off), "out": out_t, "phases": []}
         for P in phases:
+            names = sorted({x[0] for x in P["src"]})
+            at = {nm: i for i, nm in enumerate(names)}
             plan["phases"].append({
                 "split": contract.GroupedSplit(np.asarray(P["split"], dtype=np.int64), kind, dev),
                 "gemm": contract.GroupedGemm(np.asarray(P["gemm"], dtype=np.int64),
                                              np.asarray(P["alpha"], dtype=np.float64), kind, dev),
-                "src_names": [x[0] for x in P["src"]],
+                "src_names": names,
+                "src_at": np.array([at[x[0]] for x in P["src"]]),
                 "src_coef": np.stack([x[1] for x in P["src"]]),
                 "src_off": np.array([x[2] for x in P["src"]], dtype=np.int64),
             })
@@ -532,8 +537,10 @@ class QEnergy:
         org = np.array([a0, b0, c0, d0], dtype=np.int64)
         for ph in plan["phases"]:
             offs = ph["src_coef"] @ org + ph["src_off"]
-            ptrs = [base[nm].data_ptr() + int(o) * base[nm].element_size() for nm, o in zip(ph["src_names"], offs)]
-            ph["split"].run(ptrs)
+            at, ts = ph["src_at"], [base[nm] for nm in ph["src_names"]]
+            addr = np.array([t.data_ptr() for t in ts], dtype=np.int64)
+            size = np.array([t.element_size() for t in ts], dtype=np.int64)
+            ph["split"].run(addr[at] + offs * size[at])
             ph["gemm"].run(self.status)
         return plan["out"]["z"], plan["out"]["x"]
 
@@ -546,10 +553,11 @@ class QEnergy:
         t2 = t2.contiguous()
         vvooT, t2T = self._transposed(er, t2)
         for (a0, a1, b0, b1, c0, c1), dlo, dhi in self._work(group_list, d_ranges):
-            slabs = self._slabs(t3_abc, (a0, a1, b0, b1, c0, c1, c0, nv), which=("Sab", "Sac", "Sbc"))
+            slabs = {}
             for d0, d1 in self._chunks(dlo, dhi):
                 r = (a0, a1, b0, b1, c0, c1, d0, d1)
-                self._slabs(t3_abc, r, which=("Sad", "Sbd", "Scd"), out=slabs)
+                # the slabs without d once per group, with the first chunk's others
+                self._slabs(t3_abc, r, which=("Sad", "Sbd", "Scd") if slabs else _SLABS, out=slabs)
                 if self.kind is None:
                     z, x = self._run_fp64(er, t2, slabs, r)
                 else:

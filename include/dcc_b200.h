@@ -196,6 +196,12 @@ DCC_API int dcc_t3_r1(const double *t3, const double *oovv, const int32_t *ijk, 
  * src/rccsdt.c:411-561 (last record wins where records collide). */
 DCC_API int dcc_redistribute_ijk_to_abc(const double *t3_ijk, double *t3_abc, int64_t nocc, int64_t nvir, void *stream);
 
+/* The slabs target[p] = T[a0..a1, b0..b1, :, i, j, k] ([a1-a0][b1-b0][nvir][nocc]^3 each, DEVICE) of
+ * up to six ranges (a0, a1, b0, b1) = ranges[4p..4p+3] (targets and ranges HOST arrays), as
+ * dcc_fill_t3_from_abc fills one, in one launch. */
+DCC_API int dcc_fill_t3_slabs(double *const *targets, const int64_t *ranges, int nslab, int64_t nvir, int64_t nocc,
+                              const double *t3_abc, void *stream);
+
 /* target[ia][ib][c][i][j][k] (row pitch ld_b over ib) for a in [a0,a1),
  * b in [b0,b1), all c, from ABC storage t3_abc[g][x][y][z] with the occupied
  * axes permuted by the virtual ordering case.  Replaces fill_t3_from_ptr_array

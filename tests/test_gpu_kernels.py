@@ -320,6 +320,25 @@ def test_fill_t3_from_abc(C, oracle, nocc, nvir, blk):
             assert np.array_equal(host(got), want)
 
 
+@pytest.mark.parametrize("nocc,nvir", [(1, 3), (2, 5), (5, 9), (8, 6), (9, 6), (17, 3)])
+def test_fill_t3_slabs(C, nocc, nvir):
+    """Six slabs in one launch (an empty one among them, cubes of either kernel's size) equal the
+    one-slab fills, which test_fill_t3_from_abc holds against the oracle."""
+    cq = C[1]
+    rng = np.random.default_rng(nocc)
+    abc = dev(rng.standard_normal((nvir * (nvir + 1) * (nvir + 2) // 6,) + (nocc,) * 3))
+    n = nvir
+    ranges = [(0, 2, 1, n), (1, 3, 0, 1), (n - 1, n, 0, n), (0, n, 2, 3), (1, 1, 0, n), (0, 1, 0, 1)]
+    shape = lambda r: (r[1] - r[0], r[3] - r[2], nvir) + (nocc,) * 3  # noqa: E731
+    got = [torch.full(shape(r), 7.0, dtype=torch.float64, device="cuda") for r in ranges]
+    cq.fill_t3_slabs(got, ranges, nvir, nocc, abc)
+    for r, g in zip(ranges, got):
+        want = torch.zeros_like(g)
+        if g.numel():
+            cq.fill_t3_from_abc(want, *r, nvir, nocc, abc, r[3] - r[2])
+        assert torch.equal(g, want)
+
+
 @pytest.mark.parametrize("nvir", [1, 2, 5, 11])
 def test_t4_project(C, oracle, nvir):
     c4 = C[2]

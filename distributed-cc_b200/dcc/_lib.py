@@ -136,6 +136,10 @@ def call(name, *args):
 
 
 def stream_ptr(stream=None):
+    """The handle of `stream`, or of the current stream of the current device.  The latter straight
+    from the runtime: building a torch.cuda.Stream for it costs 10 us, as much as the launch."""
+    if stream is None and torch.cuda.is_initialized():
+        return c_vp(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     s = torch.cuda.current_stream() if stream is None else stream
     return c_vp(s.cuda_stream)
 

@@ -26,6 +26,7 @@
 
 #include "async_util.cuh"
 #include "dcc_common.cuh"
+#include "split_util.cuh"
 
 namespace dcc {
 
@@ -439,25 +440,6 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), TN == GN ? 1 : 2)
 }
 
 // ----------------------------------------------------------------- split kernels
-
-// x = hi + lo with hi = bf16(x), lo = bf16(x - hi).
-__device__ __forceinline__ void split_bf16(double x, __nv_bfloat16 &hi, __nv_bfloat16 &lo) {
-    hi = __float2bfloat16_rn((float)x);
-    lo = __float2bfloat16_rn((float)(x - (double)__bfloat162float(hi)));
-}
-
-// x = hi + lo with hi, lo rounded to tf32 (10 explicit mantissa bits).
-__device__ __forceinline__ float round_tf32(float f) {
-    uint32_t u = __float_as_uint(f);
-    if ((u & 0x7f800000u) == 0x7f800000u) return f;
-    u += 0x1000u;  // round half away from zero on the 13 dropped bits
-    u &= 0xffffe000u;
-    return __uint_as_float(u);
-}
-__device__ __forceinline__ void split_tf32(double x, float &hi, float &lo) {
-    hi = round_tf32((float)x);
-    lo = round_tf32((float)(x - (double)hi));
-}
 
 // Generic split of a strided FP64 operand into K-major pieces:
 //   dst[m][k0 + k] for m < M, k < kw (k >= K zero-filled) from src[mmap(m) + kmap(k)]
@@ -1242,7 +1224,9 @@ static int gemm_split3(const void *A_hi, const void *A_lo, int64_t lda, const vo
     // (two per TMEM lane quarter) double its memory parallelism; the ring then
     // is three 64-byte stages to make room for their staging buffers.
     const int esz = kind == 0 ? 2 : 4;
-    // an FP32 C always takes the wide epilogue (its only instantiation)
+    // an FP32 C takes the wide epilogue, unless it is written plainly (beta = 0) after a long
+    // contraction, whose MMAs hide a narrow one: then a fourth stage instead
+    const bool f32_long = c_f32 && beta == 0.0 && Kp >= 2048 && !narrow;
     const bool wide_epi = Kp <= 4096 || c_f32;
     const int kb = (wide_epi || narrow) ? 64 : cfg.kb_bytes;
     const int tn = narrow ? 128 : GN;
@@ -1268,6 +1252,11 @@ static int gemm_split3(const void *A_hi, const void *A_lo, int64_t lda, const vo
             return gemm_launch<0, 64, 2, 4, double, 128>(mAh, mAl, mBh, mBl, iM, iN, nkb, Cn, ep, alpha, beta, status, gm,
                                                          st);
         return gemm_launch<1, 64, 2, 4, double, 128>(mAh, mAl, mBh, mBl, iM, iN, nkb, Cn, ep, alpha, beta, status, gm, st);
+    }
+    if (f32_long) {
+        float *Cf = (float *)C;
+        if (kind == 0) return gemm_launch<0, 64, 4, 4>(mAh, mAl, mBh, mBl, iM, iN, nkb, Cf, ep, alpha, beta, status, gm, st);
+        return gemm_launch<1, 64, 4, 4>(mAh, mAl, mBh, mBl, iM, iN, nkb, Cf, ep, alpha, beta, status, gm, st);
     }
     if (c_f32) {
         float *Cf = (float *)C;

@@ -507,6 +507,107 @@ class WvvvvT3:
         return r3
 
 
+_pair_split = L.bind("dcc_t3_pair_split", [L.c_vp, L.c_int, L.c_vp, L.c_i64, L.c_i64, L.c_i64, L.c_vp, L.c_int,
+                                            L.c_vp])
+_pair_split_w = L.bind("dcc_wvvvv_pair_split", [L.c_vp, L.c_vp, L.c_vp, L.c_i64, L.c_i64, L.c_vp, L.c_int, L.c_vp,
+                                                L.c_vp])
+_pair_add = L.bind("dcc_t3_pair_add", [L.c_vp, L.c_vp, L.c_vp, L.c_i64, L.c_i64, L.c_dbl, L.c_vp])
+
+
+def pair_table(nv, Kp):
+    """d << 8 | e of the pairs d <= e in lexicographic order, 0xFFFF up to Kp (uint16)."""
+    d, e = np.triu_indices(nv)
+    out = np.full(Kp, 0xFFFF, dtype=np.uint16)
+    out[:d.size] = d << 8 | e
+    return out
+
+
+class PairWvvvvT3:
+    """W_vvvv.t3 and F_vv.t3 (the strings of WvvvvT3) for a pair-symmetric W_vvvv[x,y,d,e] =
+    W[y,x,e,d], over symmetric and antisymmetric pairs (csrc/t3_pairs.cu): two GEMMs of
+    nvir(nvir+1)/2 columns and contraction per string in place of one of nvir^2 and nvir^2, half
+    the multiplications.  F_vv's three strings are shared out evenly, (F x 1 + 1 x F) / 2 in each
+    of the three W operands.  The products accumulate in FP32 over half as long a contraction
+    and are written as they are; one pass adds all six results to r3 in FP64."""
+
+    MAX_NVIR = 112
+    SYM_TOL = 1e-14  # of max|W|, as for W_oooo's pair symmetry
+
+    def __init__(self, nblocks, nvir, kind="bf16x3", device="cuda"):
+        self.n, self.nv, self.kind, self.dev = int(nblocks), int(nvir), KIND[kind], device
+        self.rows, self.npair = self.n * self.nv, self.nv * (self.nv + 1) // 2
+        Kp = padded_k(self.npair, self.kind)
+        self.tab = torch.from_numpy(pair_table(self.nv, Kp).view(np.int16)).to(device)
+        self.t = [Split(self.rows, self.npair, self.kind, device) for _ in range(2)]  # plus, minus
+        self.w = [Split(self.npair, self.npair, self.kind, device) for _ in range(2)]
+        self.sym = torch.zeros(2, dtype=f64, device=device)
+        self.sym_host = torch.zeros(2, dtype=f64, pin_memory=True)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.own = None  # results, when the caller lends no scratch
+
+    @staticmethod
+    def worthwhile(nblocks, nvir):
+        """Whether the pair form is the faster one: from nvir = 60 on, where the products outweigh the
+        pass over the results (ms of all three strings, plain / pairs: nocc=10 nvir=90 21.5 / 13.9,
+        nocc=6 nvir=93 6.7 / 4.5, nocc=10 nvir=60 3.16 / 2.78, nocc=5 nvir=64 0.90 / 0.89; below,
+        nocc=10 nvir=56 2.27 / 2.20, nocc=10 nvir=47 1.08 / 1.30, nocc=10 nvir=30 0.36 / 0.43)."""
+        return nblocks > 0 and 60 <= nvir <= PairWvvvvT3.MAX_NVIR
+
+    def _pieces(self, pm):
+        p, m = pm
+        return (ctypes.c_void_p * 4)(p.hi.data_ptr(), p.lo.data_ptr(), m.hi.data_ptr(), m.lo.data_ptr())
+
+    def _split_t(self, t3, string):
+        L.check(_pair_split(L.ptr(t3), string, L.ptr(self.tab), self.n, self.nv, self.t[0].Kp, self._pieces(self.t),
+                            self.kind, L.stream_ptr()))
+
+    def __call__(self, r3, W, t3, alpha=1.0, F=None, scratch=None):
+        """r3 += alpha (W_vvvv.t3 + F_vv.t3) and True; False, with r3 untouched, when W lacks the pair
+        symmetry (one host read of two numbers).  scratch: a contiguous tensor whose bytes may hold
+        the FP32 results (six of rows x pairs; a buffer of this object otherwise)."""
+        for x, name in ((r3, "r3"), (t3, "t3")):
+            L.as_tensor(x, f64, name)
+        nv, rows, npair = self.nv, self.rows, self.npair
+        if r3.numel() != rows * nv * nv or t3.numel() != r3.numel() or W.numel() != nv ** 4:
+            raise ValueError("r3, t3 must be [nblocks, nvir^3] and W [nvir]^4")
+        W = L.as_tensor(W.contiguous(), f64, "W")
+        if F is not None:
+            F = L.as_tensor(F.contiguous(), f64, "F")
+            if F.numel() != nv * nv:
+                raise ValueError("F must be [nvir, nvir]")
+        self.sym.zero_()
+        L.check(_pair_split_w(L.ptr(W), L.ptr(F), L.ptr(self.tab), nv, self.w[0].Kp, self._pieces(self.w), self.kind,
+                              L.ptr(self.sym), L.stream_ptr()))
+        self.sym_host.copy_(self.sym, non_blocking=True)
+        ready = torch.cuda.Event()
+        ready.record()
+        self._split_t(t3, 0)  # the device goes on while the host looks at W's symmetry
+        ready.synchronize()
+        dev, big = float(self.sym_host[0]), float(self.sym_host[1])
+        if not dev <= self.SYM_TOL * max(big, 1e-300):
+            return False
+        need = 6 * rows * npair
+        if scratch is not None and scratch.is_contiguous() and scratch.numel() * scratch.element_size() >= 4 * need:
+            C = scratch.view(-1).view(torch.uint8)[:4 * need].view(torch.float32)
+        else:
+            if self.own is None:
+                self.own = torch.empty(need, dtype=torch.float32, device=self.dev)
+            C = self.own
+        C = C.view(3, 2, rows * npair)
+        for s in range(3):
+            if s:
+                self._split_t(t3, s)
+            for pm in range(2):
+                out = C[s, pm]
+                if s < 2:  # [q][pair][free]: the pass reads along the free index
+                    gemm_(self.w[pm], self.t[pm], out, lin(nv), two(nv, npair * nv, 1), 1.0, 0.0, self.status)
+                else:
+                    gemm_(self.t[pm], self.w[pm], out, lin(npair), lin(1), 1.0, 0.0, self.status)
+        ptr = lambda pm: (ctypes.c_void_p * 3)(*[C[s, pm].data_ptr() for s in range(3)])  # noqa: E731
+        L.check(_pair_add(ptr(0), ptr(1), L.ptr(r3), self.n, nv, float(alpha), L.stream_ptr()))
+        return True
+
+
 def wvvvv_t3_fp64_(r3, W, t3, alpha=1.0):
     """Plain FP64 GPU path of the same three einsums (cuBLAS DGEMM through torch)."""
     n, nv = t3.shape[0], t3.shape[1]

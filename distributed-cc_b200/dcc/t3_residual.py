@@ -247,6 +247,10 @@ class T3Residual:
             self.xa = contract.Split(no * nv * nv, nv, k, device)
             self.xb = contract.Split(no * no * nv, nv, k, device)
             self.wvvvv = contract.WvvvvT3(self.n3, nv, precision, device)
+            # the pair form reads W_vvvv's symmetry back to the host: not where the caller rules
+            # host reads out
+            self.pairs = contract.PairWvvvvT3(self.n3, nv, precision, device) if (
+                not woooo_pair_symmetric and contract.PairWvvvvT3.worthwhile(self.n3, nv)) else None
             self.ya = contract.Split(no * no * nv, no, k, device)
             self.yb = contract.Split(no * nv * nv, no, k, device)
             self.status = torch.zeros(1, dtype=torch.int32, device=device)
@@ -406,6 +410,9 @@ class T3Residual:
         """W_vvvv.t3 (distr_cc/rccsdt.py:421-427); in split precision F_vv.t3 rides in the same GEMMs."""
         if self.precision == "fp64":
             return contract.wvvvv_t3_fp64_(r3, d.W_vvvv, t3)
+        # S has been gathered: its buffer holds the pair results
+        if self.pairs is not None and self.pairs(r3, d.W_vvvv, t3, F=d.F_vv, scratch=self.S):
+            return r3
         return self.wvvvv(r3, d.W_vvvv, t3, F=d.F_vv)
 
     def tune(self, d, t3):
@@ -468,7 +475,8 @@ class T3Residual:
             return False
         if self.precision == "fp64":
             return True
-        return int(self.status.item()) == 0 and int(self.wvvvv.status.item()) == 0
+        return int(self.status.item()) == 0 and int(self.wvvvv.status.item()) == 0 and (
+            self.pairs is None or int(self.pairs.status.item()) == 0)
 
 
 def update_t3_(t3, r3, d, nvir_active=None, norms=None, workspace=None, write_r3=True):

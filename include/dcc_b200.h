@@ -182,6 +182,26 @@ DCC_API int dcc_t3_divide_update_noalloc(double *t3, double *r3, const double *e
                                          int64_t nblocks, int64_t nvir, int64_t nvir_active, int write_r3,
                                          double *norms, void *stream);
 
+/* W_vvvv.t3 over symmetric / antisymmetric pairs (a pair-symmetric W_vvvv[x,y,d,e] = W[y,x,e,d]):
+ * pairs: DEVICE uint16 [Kp], d << 8 | e for d <= e in lexicographic order, 0xFFFF past the
+ * nvir(nvir+1)/2 pairs; pieces: HOST array of the plus hi, plus lo, minus hi, minus lo split arrays
+ * [rows][Kp] (DEVICE; bf16 for kind 0, float for kind 1; 16-byte aligned, Kp a multiple of 8);
+ * nvir <= 112.
+ * dcc_t3_pair_split: rows (q, f) of t[d,e] +- t[e,d], t = t3[q] with its free index f last (string 0,
+ * t3[d][e][f]), in the middle (1, t3[d][f][e]) or first (2, t3[f][d][e]); the diagonal once, in plus.
+ * dcc_wvvvv_pair_split: rows x <= y of (W[x,y,d,e] +- W[x,y,e,d]) / 2, W with the F_vv strings' share
+ * (F[x,d] delta(y,e) + delta(x,d) F[y,e]) / 2 when F is not NULL; sym (DEVICE uint64[2], zeroed by
+ * the caller) receives the bits of max |W[x,y,d,e] - W[y,x,e,d]| and of max |W|.
+ * dcc_t3_pair_add: r3[q][a][b][c] += alpha (E1[a,b] + E2[a,c] + E3[b,c]), E[x,y] = plus + minus for
+ * x < y, plus - minus for x > y, plus for x = y of the unordered pair; plus[i] / minus[i] (HOST
+ * arrays of DEVICE float buffers): E1 [q][pair][c], E2 [q][pair][b], E3 [q][a][pair]. */
+DCC_API int dcc_t3_pair_split(const double *t3, int string, const uint16_t *pairs, int64_t nblocks, int64_t nvir,
+                              int64_t Kp, void *const *pieces, int kind, void *stream);
+DCC_API int dcc_wvvvv_pair_split(const double *W, const double *F, const uint16_t *pairs, int64_t nvir, int64_t Kp,
+                                 void *const *pieces, int kind, uint64_t *sym, void *stream);
+DCC_API int dcc_t3_pair_add(const float *const *plus, const float *const *minus, double *r3, int64_t nblocks,
+                            int64_t nvir, double alpha, void *stream);
+
 /* r1[nocc][nvir] += the T3 part of r1 (distr_cc/rccsdt.py:262-296) from the canonical blocks t3
  * [nblocks][nvir^3] of the triples ijk (DEVICE int32 [nblocks][3]) and oovv = <ij|ab>
  * [nocc][nocc][nvir][nvir], in one pass over t3; a block whose triple lies outside [0, nocc) adds

@@ -243,3 +243,40 @@ def test_split_of_fp32_source(C, kind, maps):
     s32 = c.Split(M, K, k).fill(X32, fm, fk)
     s64 = c.Split(M, K, k).fill(X64, fm, fk)
     assert torch.equal(s32.hi, s64.hi) and torch.equal(s32.lo, s64.lo)
+
+
+@pytest.mark.parametrize("kind", ["bf16x3", "tf32x3"])
+@pytest.mark.parametrize("nblk,nv", [(1, 1), (3, 2), (2, 7), (3, 16), (2, 31), (2, 33), (1, 64), (1, 112)])
+def test_pair_wvvvv(C, kind, nblk, nv):
+    """W_vvvv.t3 + F_vv.t3 over symmetric / antisymmetric pairs against the FP64 einsums: remainders of
+    every tile (pairs, rows, k-blocks, 32-wide column chunks) and the largest nvir; error within
+    that of the plain split form (which the tests above bound).  A W without the symmetry, or
+    with a NaN, is refused and leaves r3 alone."""
+    g = torch.Generator(device="cuda").manual_seed(nv)
+    rnd = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda", generator=g)  # noqa: E731
+    W = rnd(nv, nv, nv, nv) * 0.1
+    W = (0.5 * (W + W.permute(1, 0, 3, 2))).contiguous()
+    F, t3, r0 = rnd(nv, nv), rnd(nblk, nv, nv, nv), rnd(nblk, nv, nv, nv)
+    want = C.wvvvv_t3_fp64_(torch.zeros_like(r0), W, t3)
+    want += torch.einsum("ad,qdbc->qabc", F, t3) + torch.einsum("bd,qadc->qabc", F, t3) + \
+        torch.einsum("cd,qabd->qabc", F, t3)
+    op = C.PairWvvvvT3(nblk, nv, kind)
+    r = r0.clone()
+    assert op(r, W, t3, F=F)
+    assert int(op.status.item()) == 0
+    err = float((r - r0 - want).norm() / want.norm())
+    plain = C.WvvvvT3(nblk, nv, kind)(r0.clone(), W, t3, F=F)
+    ref = float((plain - r0 - want).norm() / want.norm())
+    # the FP32 accumulation, whose error grows with its length K, runs over nvir(nvir+1)/2 terms in
+    # place of nvir^2; the pieces' own rounding is the same
+    assert err <= 1.5 * ref + 1e-7
+    # lent scratch, and accumulation with alpha
+    r2 = r0.clone()
+    assert op(r2, W, t3, alpha=-2.0, F=F, scratch=torch.empty(6 * nblk * nv * op.npair, dtype=torch.float32, device="cuda"))
+    assert float((r2 - r0 + 2.0 * (r - r0)).abs().max()) <= 1e-6 * float(want.abs().max())
+    if nv > 1:
+        for bad in (1e-6, float("nan")):
+            Wb = W.clone()
+            Wb[0, 1, 0, 0] += bad
+            keep = r.clone()
+            assert not op(r, Wb, t3, F=F) and torch.equal(r, keep)

@@ -463,7 +463,8 @@ struct SplitWord;
 template <>
 struct SplitWord<0> {
     using T = uint32_t;
-    static __device__ __forceinline__ T make(double x) {
+    template <typename S>
+    static __device__ __forceinline__ T make(S x) {
         __nv_bfloat16 h, l;
         split_bf16(x, h, l);
         return (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
@@ -472,7 +473,8 @@ struct SplitWord<0> {
 template <>
 struct SplitWord<1> {
     using T = uint2;
-    static __device__ __forceinline__ T make(double x) {
+    template <typename S>
+    static __device__ __forceinline__ T make(S x) {
         float h, l;
         split_tf32(x, h, l);
         return make_uint2(__float_as_uint(h), __float_as_uint(l));
@@ -493,7 +495,7 @@ struct SplitArgs {
 };
 
 __device__ __forceinline__ double split_src(const double *p, int o) { return __ldg(p + o); }
-__device__ __forceinline__ double split_src(const float *p, int o) { return (double)__ldg(p + o); }
+__device__ __forceinline__ float split_src(const float *p, int o) { return __ldg(p + o); }
 
 // One warp moves one 32-row x 64-k tile (tile row ty, first column kt) with no
 // CTA-wide barrier.  Each lane holds its tile row's source address (64-bit)
@@ -535,8 +537,8 @@ __device__ __forceinline__ void split_tile(const S *__restrict__ src, const Spli
         for (int r = 0; r < SP_TM; r++) {
             const S *b = (const S *)__shfl_sync(0xffffffffu, (unsigned long long)base, r);
             const bool rv = __shfl_sync(0xffffffffu, rvalid, r);
-            const double va = (rv && koa >= 0) ? split_src(b, koa) : 0.0;
-            const double vb = (rv && kob >= 0) ? split_src(b, kob) : 0.0;
+            const S va = (rv && koa >= 0) ? split_src(b, koa) : S(0);
+            const S vb = (rv && kob >= 0) ? split_src(b, kob) : S(0);
             tile[r * SP_PITCH + lane] = SplitWord<KIND>::make(va);
             tile[r * SP_PITCH + lane + 32] = SplitWord<KIND>::make(vb);
         }
@@ -546,7 +548,7 @@ __device__ __forceinline__ void split_tile(const S *__restrict__ src, const Spli
 #pragma unroll 16
         for (int kk = 0; kk < kn; kk++) {
             const int ko = __shfl_sync(0xffffffffu, kk < 32 ? koa : kob, kk & 31);
-            const double v = (rvalid && ko >= 0) ? split_src(base, ko) : 0.0;
+            const S v = (rvalid && ko >= 0) ? split_src(base, ko) : S(0);
             tile[lane * SP_PITCH + kk] = SplitWord<KIND>::make(v);
         }
     }

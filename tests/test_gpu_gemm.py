@@ -280,3 +280,24 @@ def test_pair_wvvvv(C, kind, nblk, nv):
             Wb[0, 1, 0, 0] += bad
             keep = r.clone()
             assert not op(r, Wb, t3, F=F) and torch.equal(r, keep)
+
+
+@pytest.mark.parametrize("kind", ["bf16x3", "tf32x3"])
+def test_split_fp32_source(C, kind):
+    """An FP32 source gives the pieces of the same values as doubles, bit for bit: every exponent,
+    ties of both roundings, denormals, the largest values (hi rounds to infinity), infinities
+    and NaN."""
+    import numpy as np
+    k = C.KIND[kind]
+    rng = np.random.default_rng(5)
+    u = rng.integers(0, 1 << 32, 1 << 16, dtype=np.uint64).astype(np.uint32)
+    u[:4096] = (u[:4096] & 0xFFFF0000) | 0x8000  # ties of bf16
+    u[4096:8192] = (u[4096:8192] & 0xFFFFE000) | 0x1000  # ties of tf32
+    u[8192:8200] = [0x7F800000, 0xFF800000, 0x7FC00000, 0x7F7FFFFF, 0xFF7FFFFF, 1, 0x807FFFFF, 0]
+    f = torch.from_numpy(u.view(np.float32).reshape(256, 256)).cuda()
+    a = C.Split(256, 256, k, "cuda").fill(f, C.lin(256), C.lin(1))
+    b = C.Split(256, 256, k, "cuda").fill(f.double(), C.lin(256), C.lin(1))
+    bits = torch.int16 if k == 0 else torch.int32
+    for x, y in ((a.hi, b.hi), (a.lo, b.lo)):
+        nan = torch.isnan(x) & torch.isnan(y)
+        assert bool(((x.view(bits) == y.view(bits)) | nan).all())

@@ -143,6 +143,17 @@ def t4_add_(t4, r4, nocc4, nvir):
     return t4
 
 
+def t4_w_oooovv(Ts, E, nocc, nvir, alpha=1.0):
+    """alpha sum_{i,f,e} E[m,i,e,f] Ts[i,j,k,l,f,a,b,e] as [j,k,l,m,a,b]: the T4 part of W_oooovv from
+    P4_201 of every ordering, read in place."""
+    Ts, E = L.as_tensor(Ts, f64, "Ts"), L.as_tensor(E, f64, "E")
+    if Ts.numel() != (nocc * nvir) ** 4 or E.numel() != (nocc * nvir) ** 2:
+        raise ValueError("Ts must be [nocc^4, nvir^4] and E [nocc, nocc, nvir, nvir]")
+    out = torch.empty((nocc,) * 4 + (nvir,) * 2, dtype=f64, device=Ts.device)
+    L.call("dcc_t4_w_oooovv", L.ptr(Ts), L.ptr(E), L.ptr(out), nocc, nvir, float(alpha), L.stream_ptr())
+    return out
+
+
 def t4_strings(ops, desc, quads, nocc, nvir, r4, beta=0.0, status=None, pairs=None):
     """r4 = beta r4 + every string of the descriptor table `desc` [nstr, 32] (int64, device)
     over every stored block of `quads` [nq, 4] (int32, device), one launch (the per-block

@@ -72,6 +72,7 @@ _SIGS = {
     "dcc_fill_t3_from_abc": [c_vp] + [c_i64] * 6 + [c_vp, c_i64, c_vp],
     "dcc_t4_project_1_minus_p4_p31_inplace": [c_vp, c_i64, c_i64, c_dbl, c_dbl, c_vp],
     "dcc_t4_spin_summation_inplace": [c_vp, c_i64, c_i64, c_str, c_dbl, c_dbl, c_vp],
+    "dcc_t4_w_oooovv": [c_vp, c_vp, c_vp, c_i64, c_i64, c_dbl, c_vp],
     "dcc_t4_unpack_all": [c_vp] * 5 + [c_i64, c_i64, c_vp],
     "dcc_t4_transpose_add": [c_vp, c_vp, c_i64, c_vp],
     "dcc_t4_spin_summation_quadruple_sym": [c_vp] * 5 + [c_i64, c_vp],

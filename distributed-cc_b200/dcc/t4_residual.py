@@ -213,6 +213,40 @@ def _einsum(kind, subs, X, Y, out, alpha):
         contract.einsum_into(subs, X, Y, out, alpha, 1.0, kind)
 
 
+def _t4_part_fits(nocc, nv):
+    """The strings kernel takes W_oovvvv's T4 part: its accumulator and operand limits."""
+    from . import _c_rccsdtq
+    return _c_rccsdtq.t4_strings_rows_per_cta(nocc * nocc, nv) >= 1 and (nocc * nv) ** 4 < 1 << 31
+
+
+def _t4_parts(E, T4s, nocc, nv):
+    """The T4 parts of W_oooovv [j,k,l,m,a,b] and W_oovvvv [k,l,a,b,c,e] (distr_cc/rccsdtq.py:756-775)
+    from P4_201 of every ordering, read in place (an einsum's transposed copies of it took 0.92 ms
+    at nocc=7 / nvir=11, the two products here 0.34 ms, 1.1 with the einsums).  W_oovvvv's is one string of the strings
+    kernel over "blocks" (k, l): rows e, columns a, b, c, summed over f and the pair (i, j)."""
+    from . import _c_rccsdtq
+
+    def build():
+        n2, V = nocc * nocc, nv ** 4
+        d = [0] * 32
+        d[8], d[9] = nocc * V, V  # T4s at the block's occupied indices: its third and fourth slots hold k, l
+        d[15] = nv  # the pair operand [(i, j)][e][f]: row letter e in output position d
+        d[16], d[17], d[18] = nv * nv, nv, 1  # T4s [(i, j)][k][l][f][a][b][c]
+        d[1], d[20] = 1, 8
+        d[21:24] = nv, 1, nv ** 3  # f
+        d[24:27] = n2, nv * nv, n2 * V  # (i, j)
+        d[27] = struct.unpack("<q", struct.pack("<d", -0.5))[0]
+        d[28], d[29] = 4, 1 | 2 << 4 | 3 << 8
+        quads = [(0, 0, k, l) for k in range(nocc) for l in range(nocc)]
+        return torch.tensor([d], dtype=torch.int64, device=E.device), torch.tensor(quads, dtype=torch.int32,
+                                                                                   device=E.device)
+    desc, quads = _cached(("t4_part", nocc, nv), E.device, build)
+    Word = torch.empty((nocc * nocc, nv ** 4), dtype=f64, device=E.device)
+    _c_rccsdtq.t4_strings([E.transpose(0, 1).contiguous(), T4s], desc, quads, nocc, nv, Word, 0.0,
+                          fused_status(E.device))
+    return _c_rccsdtq.t4_w_oooovv(T4s, E, nocc, nv, 0.5), Word.view((nocc,) * 2 + (nv,) * 4)
+
+
 def build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spin4, T4full=None, T4s=None):
     """The W builders of distr_cc/rccsdtq.py:700-833 as full tensors (FP64, torch).  T4full:
     unpack_all_orderings(t4) when the caller has it already; T4s: P4_201 of every block of it."""
@@ -232,8 +266,11 @@ def build_intermediates(eris, W_oooo, W_ovov, W_vvvv, t2, t3, t3p, t4, nocc, spi
     if T4s is None:
         T4s = unpack_all_orderings(t4, nocc) if T4full is None else T4full.clone()
         spin4(T4s)
-    Woo = 0.5 * e('mief,ijklfabe->jklmab', eris[o, o, v, v], T4s)
-    Word = -0.5 * e('jief,ijklfabc->klabce', eris[o, o, v, v], T4s)
+    if T4s.is_cuda and T4s.is_contiguous() and _t4_part_fits(nocc, t2.shape[2]):
+        Woo, Word = _t4_parts(eris[o, o, v, v].contiguous(), T4s, nocc, t2.shape[2])
+    else:
+        Woo = 0.5 * e('mief,ijklfabe->jklmab', eris[o, o, v, v], T4s)
+        Word = -0.5 * e('jief,ijklfabc->klabce', eris[o, o, v, v], T4s)
     del T4s
     Woo = Woo + e('amef,ijkebf->ijkmab', eris[v, o, v, v], t3)
     c_t2 = 2.0 * t2 - t2.permute(0, 1, 3, 2)

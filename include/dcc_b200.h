@@ -370,6 +370,12 @@ DCC_API int dcc_t4_strings(const double *const *ops, const int64_t *op_numel, in
 /* Output rows a per CTA that dcc_t4_strings uses for nq blocks (-1: nvir too large). */
 DCC_API int dcc_t4_strings_rows_per_cta(int64_t nq, int64_t nvir);
 
+/* out[j][k][l][m][a][b] = alpha sum_{i,f,e} E[m][i][e][f] Ts[i][j][k][l][f][a][b][e]: the T4 part of W_oooovv
+ * (distr_cc/rccsdtq.py:756-775) from Ts, P4_201 of every ordering (dcc_t4_unpack_all), and
+ * E = <mi|ef>; all DEVICE, nocc and nvir below 1024. */
+DCC_API int dcc_t4_w_oooovv(const double *Ts, const double *E, double *out, int64_t nocc, int64_t nvir, double alpha,
+                            void *stream);
+
 /* r4[q] /= eia[i,a]+eia[j,b]+eia[k,c]+eia[l,d] for ijkl = local_ijkl[q]
  * (DEVICE int32 [nlocal][4]).  Replaces r4_local_tri_divide_e_
  * (src/rccsdtq.c:1055-1088). */

@@ -184,6 +184,26 @@ def test_unpack_all_orderings(no, nv):
     assert torch.equal(Ts.view(no ** 4, -1), ws)
 
 
+@pytest.mark.parametrize("no,nv", [(1, 1), (2, 3), (3, 4), (9, 2), (4, 9), (2, 13)])
+def test_t4_parts(no, nv):
+    """The T4 parts of W_oooovv and W_oovvvv by the matrix-pipe kernels against the einsums (fewer
+    and more than one tile of m and of (a, b), contractions that end inside a step of four;
+    1e-13 of the largest entry: sums of at most nocc^2 nvir^2 products in another order)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from dcc import t4_residual as tr
+    g = torch.Generator(device="cuda").manual_seed(no)
+    E = torch.randn((no, no, nv, nv), dtype=torch.float64, device="cuda", generator=g)
+    T = torch.randn((no,) * 4 + (nv,) * 4, dtype=torch.float64, device="cuda", generator=g)
+    assert tr._t4_part_fits(no, nv)
+    got = tr._t4_parts(E, T, no, nv)
+    want = (0.5 * torch.einsum('mief,ijklfabe->jklmab', E, T), -0.5 * torch.einsum('jief,ijklfabc->klabce', E, T))
+    torch.cuda.synchronize()
+    assert int(tr.fused_status("cuda").item()) == 0
+    for x, y in zip(got, want):
+        assert float((x - y).abs().max()) <= 1e-13 * float(y.abs().max())
+
+
 @pytest.mark.parametrize("no,nv", [(3, 1), (3, 2), (3, 8), (4, 9), (5, 7), (6, 4), (4, 20)])
 def test_fused_strings_tiles(no, nv):
     """The tile shapes of the strings kernel (one row or column, fewer than one 8 x 8 tile, whole

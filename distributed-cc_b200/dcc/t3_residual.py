@@ -271,7 +271,52 @@ class T3Residual:
                     self.wooa = contract.Split(no * no, kind=k, device=device, pieces=self.woo_pieces)
                     self.woob = contract.Split(no * nv ** 3, kind=k, device=device, pieces=self.woo_pieces)
 
+        self._small = None
+        if precision != "fp64" and torch.device(device).type == "cuda":
+            self._small = self._small_split()
+
     # ------------------------------------------------------------ pieces
+    def _small_split(self):
+        """One grouped split for the operands of the S GEMMs made from t2 and the W intermediates
+        (seven launches of a few us of work each otherwise), in the order _s_split lists them."""
+        no, nv, c, pl = self.no, self.nv, contract, self.plan
+        ops = [(self.ya, 0, c.three(nv, no, no, 1, no ** 3), c.lin(no * no)),
+               (self.yb, 0, c.lin(1), c.lin(no * nv * nv)),
+               (self.xa, 0) + pl["x"]["a"][0][1:], (self.xb, 0) + pl["x"]["b"][0][1:]]
+        if self.with_oo:
+            ops += [(self.ooa, i) + pl["oo"]["a"][i][1:] for i in range(2)] + [(self.t1a, 0) + pl["t1"]["a"][0][1:]]
+        spec = []
+        for op, i, fm, fk in ops:
+            off, k, w = op.pieces[i]
+            spec.append([op.hi.data_ptr(), op.lo.data_ptr(), op.M, k, w, op.Kp, off] + list(c.as4(fm)) + list(c.as4(fk))
+                        + [0])
+        return c.GroupedSplit(spec, self.kind, self.dev)
+
+    def _fill_small(self, d):
+        """The operands of _small_split from d's tensors; returns the OO sources it made."""
+        no, nv = self.no, self.nv
+        src = {}
+        srcs = [(d.W_vooo, nv * no ** 3), (d.t2, (no * nv) ** 2), (d.W_vvvo, nv ** 3 * no), (d.t2, (no * nv) ** 2)]
+        if self.with_oo:
+            src = {"G2": (-0.5 * (d.W_ovov + d.W_ovvo.permute(0, 1, 3, 2))).permute(2, 1, 0, 3).contiguous(),
+                   "Wvo_half": 0.5 * d.W_ovvo, "W_ovov": d.W_ovov}
+            srcs += [(src[n], (no * nv) ** 2) for n in ("G2", "Wvo_half", "W_ovov")]
+        if self._small is not None and all(t.dtype == f64 and t.is_cuda and t.is_contiguous() and t.numel() == n
+                                           for t, n in srcs):
+            self._small.run([t.data_ptr() for t, _ in srcs])
+            return
+        # other layouts and types: one by one, each through its own checks
+        c, pl = contract, self.plan
+        self.ya.fill(d.W_vooo, c.three(nv, no, no, 1, no ** 3), c.lin(no * no))
+        self.yb.fill(d.t2, c.lin(1), c.lin(no * nv * nv))
+        self.xa.fill(d.W_vvvo, *pl["x"]["a"][0][1:])
+        self.xb.fill(d.t2, *pl["x"]["b"][0][1:])
+        if self.with_oo:
+            for i, (name, fm, fk) in enumerate(pl["oo"]["a"]):
+                self.ooa.fill_piece(i, src[name], fm, fk)
+            name, fm, fk = pl["t1"]["a"][0]
+            self.t1a.fill(src[name], fm, fk)
+
     def _gemm(self, name, A, B, C, frow, fcol, alpha, beta, Kp=None):
         """One of the S GEMMs under the tile and raster configuration tuned for it (tune()); its
         arguments are kept so that tune() can time it alone."""
@@ -351,21 +396,14 @@ class T3Residual:
         no, nv = self.no, self.nv
         S = self.S
         x = pl["x"]
+        self._fill_small(d)
         self._y_into_s(d)  # writes S first
-        self.xa.fill(d.W_vvvo, *x["a"][0][1:])
-        self.xb.fill(d.t2, *x["b"][0][1:])
         self._gemm("x", self.xa, self.xb, S, *x["out"], x["alpha"], 1.0)
         if not self.with_oo:
             return
-        src = {"G2": (-0.5 * (d.W_ovov + d.W_ovvo.permute(0, 1, 3, 2))).permute(2, 1, 0, 3).contiguous(),
-               "Wvo_half": 0.5 * d.W_ovvo, "W_ovov": d.W_ovov, "U": self.U}
         oo, t1 = pl["oo"], pl["t1"]
-        for i, (name, fm, fk) in enumerate(oo["a"]):
-            self.ooa.fill_piece(i, src[name], fm, fk)
-        for i, (name, fm, fk) in enumerate(oo["b"]):
-            self.oob.fill_piece(i, src[name], fm, fk)
-        name, fm, fk = t1["a"][0]
-        self.t1a.fill(src[name], fm, fk)
+        for i, (_, fm, fk) in enumerate(oo["b"]):
+            self.oob.fill_piece(i, self.U, fm, fk)
         self._gemm("oo", self.ooa, self.oob, S, *oo["out"], oo["alpha"], oo["beta"])
         self._gemm("t1", self.t1a, self.oob, S, *t1["out"], t1["alpha"], t1["beta"], Kp=self.t1a.Kp)
 

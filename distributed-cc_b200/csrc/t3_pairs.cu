@@ -298,6 +298,47 @@ __global__ void __launch_bounds__(PR_THREADS, 2) k_pair_add(PairC C, double *__r
     }
 }
 
+// The small matrices of the residual's OO contractions in one launch (some fifteen element-wise
+// launches otherwise, most of the host time of a small molecule's residual):
+//   G2[i,a,l,d] = -(W_ovov[l,a,i,d] + W_ovvo[l,a,d,i]) / 2,   Wh = W_ovvo / 2,
+//   A[(i,j)][(l,m)] = (W_oooo[l,m,i,j] - F_oo[l,i] delta(m,j)) / 2,
+// and the bits of max |W_oooo[l,m,i,j] - W_oooo[m,l,j,i]| / 2 and max |W_oooo| in sym[0..1] (zeroed
+// by the caller), by which the caller decides whether A stands for W_oooo.
+__global__ void __launch_bounds__(256) k_oo_small(const double *__restrict__ Wov, const double *__restrict__ Wvo,
+                                                  const double *__restrict__ Woo, const double *__restrict__ F, int no,
+                                                  int nv, double *__restrict__ G2, double *__restrict__ Wh,
+                                                  double *__restrict__ A, unsigned long long *sym) {
+    const int64_t n1 = (int64_t)no * no * nv * nv, n2 = (int64_t)no * no * no * no;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t e = first; e < n1; e += step) {
+        Wh[e] = 0.5 * Wvo[e];
+        const int d = (int)(e % nv), l = (int)((e / nv) % no), a = (int)((e / ((int64_t)nv * no)) % nv),
+                  i = (int)(e / ((int64_t)nv * no * nv));
+        const int64_t la = (int64_t)l * nv + a;
+        G2[e] = -0.5 * (Wov[(la * no + i) * nv + d] + Wvo[(la * nv + d) * no + i]);
+    }
+    unsigned long long dev = 0, big = 0;
+    for (int64_t e = first; e < n2; e += step) {
+        const int m = (int)(e % no), l = (int)((e / no) % no), j = (int)((e / ((int64_t)no * no)) % no),
+                  i = (int)(e / ((int64_t)no * no * no));
+        const double w = Woo[(((int64_t)l * no + m) * no + i) * no + j], wt = Woo[(((int64_t)m * no + l) * no + j) * no + i];
+        A[e] = 0.5 * w - (m == j ? 0.5 * F[l * no + i] : 0.0);
+        const unsigned long long x = (unsigned long long)__double_as_longlong(fabs(0.5 * (w - wt))),
+                                 y = (unsigned long long)__double_as_longlong(fabs(w));
+        dev = x > dev ? x : dev;
+        big = y > big ? y : big;
+    }
+    for (int k = 16; k > 0; k >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, dev, k), y = __shfl_xor_sync(0xffffffffu, big, k);
+        dev = x > dev ? x : dev;
+        big = y > big ? y : big;
+    }
+    if ((threadIdx.x & 31) == 0 && big != 0) {  // a warp without elements adds nothing
+        atomicMax(sym, dev);
+        atomicMax(sym + 1, big);
+    }
+}
+
 template <typename K>
 static void pair_smem(K kern, size_t bytes) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -398,4 +439,18 @@ extern "C" int dcc_t3_pair_add(const float *const *plus, const float *const *min
     pair_smem(k_pair_add, smem);
     k_pair_add<<<(unsigned)(nblocks * nvir), PR_THREADS, smem, as_stream(stream)>>>(C, r3, nv, np, alpha);
     return launch_status("t3_pair_add");
+}
+
+extern "C" int dcc_t3_oo_operands(const double *W_ovov, const double *W_ovvo, const double *W_oooo, const double *F_oo,
+                                  int64_t nocc, int64_t nvir, double *G2, double *Wvo_half, double *A, uint64_t *sym,
+                                  void *stream) {
+    clear_error();
+    DCC_REQUIRE(nocc >= 0 && nvir >= 0 && nocc < 4096 && nvir < 4096, DCC_ERR_SHAPE, "bad size");
+    if (nocc == 0 || nvir == 0) return DCC_OK;
+    DCC_REQUIRE(W_ovov && W_ovvo && W_oooo && F_oo && G2 && Wvo_half && A && sym, DCC_ERR_NULL, "NULL buffer");
+    const int64_t n1 = nocc * nocc * nvir * nvir, n2 = nocc * nocc * nocc * nocc, n = n1 > n2 ? n1 : n2;
+    const unsigned grid = ceil_div(n, 256);
+    k_oo_small<<<grid < 148 * 8 ? grid : 148 * 8, 256, 0, as_stream(stream)>>>(
+        W_ovov, W_ovvo, W_oooo, F_oo, (int)nocc, (int)nvir, G2, Wvo_half, A, (unsigned long long *)sym);
+    return launch_status("t3_oo_operands");
 }

@@ -217,6 +217,10 @@ def woooo_foo_matrix(W_oooo, F_oo, sym_tol=1e-14, assume_symmetric=False):
     return A.reshape(no * no, no * no).contiguous(), (Wa.contiguous() if anti else None)
 
 
+_oo_operands = L.bind("dcc_t3_oo_operands", [L.c_vp] * 4 + [L.c_i64, L.c_i64] + [L.c_vp] * 5)
+SYM_TOL = 1e-14  # of max|W_oooo|: the antisymmetric part below which W_oooo has the pair symmetry
+
+
 class T3Residual:
     """compute_r3_tri for all canonical blocks of one rank."""
 
@@ -271,7 +275,7 @@ class T3Residual:
                     self.wooa = contract.Split(no * no, kind=k, device=device, pieces=self.woo_pieces)
                     self.woob = contract.Split(no * nv ** 3, kind=k, device=device, pieces=self.woo_pieces)
 
-        self._small = None
+        self._small = self._A = self._sym = None
         if precision != "fp64" and torch.device(device).type == "cuda":
             self._small = self._small_split()
 
@@ -292,14 +296,41 @@ class T3Residual:
                         + [0])
         return c.GroupedSplit(spec, self.kind, self.dev)
 
+    def _oo_sources(self, d):
+        """{G2, Wvo_half, W_ovov} of the OO GEMMs and, on a CUDA device with d's tensors laid out
+        plainly, self._A / self._sym for the W_oooo / F_oo one, all in one launch."""
+        no, nv = self.no, self.nv
+        self._A = None
+        ins = [(d.W_ovov, (no * nv) ** 2), (d.W_ovvo, (no * nv) ** 2), (d.W_oooo, no ** 4), (d.F_oo, no * no)]
+        if self._small is None or not all(t.dtype == f64 and t.is_cuda and t.is_contiguous() and t.numel() == n
+                                          for t, n in ins):
+            return {"G2": (-0.5 * (d.W_ovov + d.W_ovvo.permute(0, 1, 3, 2))).permute(2, 1, 0, 3).contiguous(),
+                    "Wvo_half": 0.5 * d.W_ovvo, "W_ovov": d.W_ovov}
+        g2, wh = torch.empty_like(d.W_ovov), torch.empty_like(d.W_ovvo)
+        self._A = torch.empty((no * no, no * no), dtype=f64, device=g2.device)
+        self._sym = torch.zeros(2, dtype=f64, device=g2.device)
+        L.check(_oo_operands(*[L.ptr(t) for t, _ in ins], no, nv, L.ptr(g2), L.ptr(wh), L.ptr(self._A),
+                             L.ptr(self._sym), L.stream_ptr()))
+        return {"G2": g2, "Wvo_half": wh, "W_ovov": d.W_ovov}
+
+    def _woooo(self, d):
+        """woooo_foo_matrix(d.W_oooo, d.F_oo) of the split path, from _oo_sources where it made it."""
+        A, self._A = self._A, None
+        if A is not None and not self.woooo_pair_symmetric:
+            dev, big = self._sym.tolist()
+            if not dev <= SYM_TOL * max(big, 1e-300):
+                A = None  # the antisymmetric part goes its own way
+        if A is not None:
+            return A, None
+        return woooo_foo_matrix(d.W_oooo, d.F_oo, SYM_TOL, assume_symmetric=self.woooo_pair_symmetric)
+
     def _fill_small(self, d):
         """The operands of _small_split from d's tensors; returns the OO sources it made."""
         no, nv = self.no, self.nv
         src = {}
         srcs = [(d.W_vooo, nv * no ** 3), (d.t2, (no * nv) ** 2), (d.W_vvvo, nv ** 3 * no), (d.t2, (no * nv) ** 2)]
         if self.with_oo:
-            src = {"G2": (-0.5 * (d.W_ovov + d.W_ovvo.permute(0, 1, 3, 2))).permute(2, 1, 0, 3).contiguous(),
-                   "Wvo_half": 0.5 * d.W_ovvo, "W_ovov": d.W_ovov}
+            src = self._oo_sources(d)
             srcs += [(src[n], (no * nv) ** 2) for n in ("G2", "Wvo_half", "W_ovov")]
         if self._small is not None and all(t.dtype == f64 and t.is_cuda and t.is_contiguous() and t.numel() == n
                                            for t, n in srcs):
@@ -357,7 +388,8 @@ class T3Residual:
         else:
             self._s_split(d)
         if self.with_oo:
-            A, Wa = woooo_foo_matrix(d.W_oooo, d.F_oo, assume_symmetric=self.woooo_pair_symmetric)
+            A, Wa = (woooo_foo_matrix(d.W_oooo, d.F_oo, assume_symmetric=self.woooo_pair_symmetric)
+                     if self.precision == "fp64" else self._woooo(d))
             if self.precision == "fp64":
                 S.view(no * no, -1).addmm_(A, self.U.view(no * no, -1))
             else:

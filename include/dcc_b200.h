@@ -202,6 +202,14 @@ DCC_API int dcc_wvvvv_pair_split(const double *W, const double *F, const uint16_
 DCC_API int dcc_t3_pair_add(const float *const *plus, const float *const *minus, double *r3, int64_t nblocks,
                             int64_t nvir, double alpha, void *stream);
 
+/* The small matrices of the residual's OO contractions (distr_cc/rccsdt.py:435-732), all DEVICE:
+ * G2[i,a,l,d] = -(W_ovov[l,a,i,d] + W_ovvo[l,a,d,i]) / 2, Wvo_half = W_ovvo / 2,
+ * A[(i,j)][(l,m)] = (W_oooo[l,m,i,j] - F_oo[l,i] delta(m,j)) / 2; sym (uint64[2], zeroed by the
+ * caller) receives the bits of max |W_oooo[l,m,i,j] - W_oooo[m,l,j,i]| / 2 and of max |W_oooo|. */
+DCC_API int dcc_t3_oo_operands(const double *W_ovov, const double *W_ovvo, const double *W_oooo, const double *F_oo,
+                               int64_t nocc, int64_t nvir, double *G2, double *Wvo_half, double *A, uint64_t *sym,
+                               void *stream);
+
 /* r1[nocc][nvir] += the T3 part of r1 (distr_cc/rccsdt.py:262-296) from the canonical blocks t3
  * [nblocks][nvir^3] of the triples ijk (DEVICE int32 [nblocks][3]) and oovv = <ij|ab>
  * [nocc][nocc][nvir][nvir], in one pass over t3; a block whose triple lies outside [0, nocc) adds

@@ -221,3 +221,38 @@ def test_woooo_split_in_k_pieces(mods, precision):
     scale = want.abs().max()
     assert float((b - want).abs().max() / scale) < TOL[precision]
     assert float((b - a).abs().max() / scale) < 1e-6
+
+
+@pytest.mark.parametrize("no,nv", [(1, 1), (2, 7), (5, 3), (9, 33)])
+def test_oo_operands(no, nv):
+    """The one-launch OO matrices equal the element-wise ones (==: the same operations), and the
+    symmetry words tell a pair-symmetric W_oooo from another and from one with a NaN."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from dcc import t3_residual as t
+    g = torch.Generator(device="cuda").manual_seed(no)
+    r = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda", generator=g)  # noqa: E731
+    res = t.T3Residual(no, nv, "bf16x3")
+
+    class D:
+        W_ovov, W_ovvo, W_oooo, F_oo = r(no, nv, no, nv), r(no, nv, nv, no), r(no, no, no, no), r(no, no)
+
+    d = D()
+    for case in ("symmetric", "plain", "nan"):
+        if case == "symmetric":
+            d.W_oooo = 0.5 * (d.W_oooo + d.W_oooo.permute(1, 0, 3, 2)).contiguous()
+        elif case == "plain":
+            d.W_oooo = r(no, no, no, no)
+        else:
+            d.W_oooo[-1, 0, 0, 0] = float("nan")
+        src = res._oo_sources(d)
+        assert torch.equal(src["G2"], (-0.5 * (d.W_ovov + d.W_ovvo.permute(0, 1, 3, 2))).permute(2, 1, 0, 3))
+        assert torch.equal(src["Wvo_half"], 0.5 * d.W_ovvo)
+        if case == "nan":
+            dev, big = res._sym.tolist()
+            assert dev != dev and big != big
+            continue
+        A, Wa = res._woooo(d)
+        want, wa = t.woooo_foo_matrix(d.W_oooo, d.F_oo)
+        assert torch.equal(A, want) and (Wa is None) == (wa is None)
+        assert (Wa is None) == (case == "symmetric" or no == 1)

@@ -205,6 +205,19 @@ def t3_r1_(r1, t3, oovv, ijk, nocc):
     return r1
 
 
+def t3_r2_fock_(r2, X, fock_ov, nocc, nvir, alpha):
+    """r2 [y,z,b,c] += alpha sum_{x,a} fock_ov[x,a] X[x,y,z,a,b,c] in FP64 (X FP64 or FP32)."""
+    if X.dtype not in (f64, torch.float32):
+        raise TypeError("X must be float64 or float32")
+    X = L.as_tensor(X, X.dtype, "X")
+    r2, fock_ov = L.as_tensor(r2, f64, "r2"), L.as_tensor(fock_ov, f64, "fock_ov")
+    if X.numel() != (nocc * nvir) ** 3 or r2.numel() != (nocc * nvir) ** 2 or fock_ov.numel() != nocc * nvir:
+        raise ValueError("X must be [nocc^3, nvir^3], r2 [nocc^2, nvir^2], fock_ov [nocc, nvir]")
+    L.call("dcc_t3_r2_fock", L.ptr(X), int(X.dtype == torch.float32), L.ptr(fock_ov), L.ptr(r2), nocc, nvir,
+           float(alpha), L.stream_ptr())
+    return r2
+
+
 def redistribute_ijk_to_abc(t3_ijk, nocc, nvir, out=None):
     """T3[i<=j<=k][abc] -> T3[a<=b<=c][ijk] at one rank
     (distr_cc/distribute_t3.py:1544-1642 with src/rccsdt.c:411-561)."""

@@ -65,6 +65,7 @@ _SIGS = {
     "dcc_fill_local_data_ijk": [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_vp],
     "dcc_r3_tri_divide_e": [c_vp, c_vp, c_vp, c_i64, c_i64, c_vp],
     "dcc_t3_divide_update": [c_vp, c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_int, c_vp, c_vp, c_size, c_vp],
+    "dcc_t3_r2_fock": [c_vp, c_int, c_vp, c_vp, c_i64, c_i64, c_dbl, c_vp],
     "dcc_t3_r1": [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_size, c_vp],
     "dcc_t3_r1_workspace_bytes": [c_i64, c_i64, c_i64],
     "dcc_redistribute_ijk_to_abc": [c_vp, c_vp, c_i64, c_i64, c_vp],

@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _c_rccsdt
 from . import t3_feedback as fb
 from .diis import DIIS
 from .synthetic import canonical_ijk
@@ -69,22 +70,24 @@ class T3Iteration:
         else:
             # all four strings here, two splits of X between them; the W parts wait in dW for
             # feedback_w (the host builds W_vooo / W_vvvo in between)
-            dr2.view(no * no, nv * nv).add_(self._fock_term(fock_ov), alpha=0.5)
+            self._fock_term_(dr2, fock_ov)
             self._dW = (torch.zeros((nv, no, no, no), dtype=f64, device=self.dev),
                         torch.zeros((nv, nv, nv, no), dtype=f64, device=self.dev))
             self.sfb.run(self._X, {"vovv": vovv, "ooov": ooov, "oovv": oovv},
                          {"r2": dr2, "W_vooo": self._dW[0], "W_vvvo": self._dW[1]})
         return dr1, dr2
 
-    def _fock_term(self, fock_ov):
-        """sum_{x,a} f[x,a] X[x,y,z,a,b,c] as [(y,z), (b,c)], summed over x in FP64 (each x's
-        product in X's type)."""
+    def _fock_term_(self, dr2, fock_ov):
+        """dr2 += 1/2 sum_{x,a} f[x,a] X[x,y,z,a,b,c], summed in FP64."""
         no, nv = self.no, self.nv
-        out = torch.zeros((no * no, nv * nv), dtype=f64, device=self.dev)
+        if no * nv <= 6144 and no < 256:
+            _c_rccsdt.t3_r2_fock_(dr2, self._X, fock_ov.to(f64).contiguous(), no, nv, 0.5)
+            return
         f = fock_ov.to(self._X.dtype)
         for x in range(no):
-            out += torch.matmul(f[x].view(1, 1, nv), self._X[x].reshape(no * no, nv, nv * nv)).view(no * no, nv * nv)
-        return out
+            dr2.view(no * no, nv * nv).add_(
+                torch.matmul(f[x].view(1, 1, nv), self._X[x].reshape(no * no, nv, nv * nv)).view(no * no, nv * nv),
+                alpha=0.5)
 
     def feedback_w(self, W_vooo, W_vvvo, oovv):
         """W_vooo, W_vvvo += their T3 parts (distr_cc/rccsdt.py:323-366), in place, from the X of

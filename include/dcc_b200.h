@@ -210,6 +210,11 @@ DCC_API int dcc_t3_oo_operands(const double *W_ovov, const double *W_ovvo, const
                                int64_t nocc, int64_t nvir, double *G2, double *Wvo_half, double *A, uint64_t *sym,
                                void *stream);
 
+/* r2[y,z,b,c] += alpha sum_{x,a} fock_ov[x,a] X[x,y,z,a,b,c] (distr_cc/rccsdt.py:300-316), FP64; X
+ * [nocc]^3[nvir]^3 double, or float when x_f32; nocc * nvir at most 6144; all DEVICE. */
+DCC_API int dcc_t3_r2_fock(const void *X, int x_f32, const double *fock_ov, double *r2, int64_t nocc, int64_t nvir,
+                           double alpha, void *stream);
+
 /* r1[nocc][nvir] += the T3 part of r1 (distr_cc/rccsdt.py:262-296) from the canonical blocks t3
  * [nblocks][nvir^3] of the triples ijk (DEVICE int32 [nblocks][3]) and oovv = <ij|ab>
  * [nocc][nocc][nvir][nvir], in one pass over t3; a block whose triple lies outside [0, nocc) adds

@@ -75,3 +75,18 @@ def test_r1_kernel(mods, no, nv):
     got = fb.r1_add_t3_(r1.cuda(), None, t3.cuda(), ijk.cuda(), no, oovv=E.cuda())
     scale = max(float((want - r1).abs().max()), float(r1.abs().max()))
     assert float((got.cpu() - want).abs().max()) <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("no,nv", [(1, 1), (2, 16), (3, 17), (5, 7)])
+def test_r2_fock(mods, dtype, no, nv):
+    """The one-launch Fock term (fewer and more than one CTA of (b, c) per (y, z)) against the
+    einsum of the same values in FP64 (1e-13: sums of nocc nvir products in another order)."""
+    from dcc import _c_rccsdt
+    g = torch.Generator(device="cuda").manual_seed(nv)
+    X = torch.randn((no,) * 3 + (nv,) * 3, dtype=torch.float64, device="cuda", generator=g).to(dtype)
+    f = torch.randn(no, nv, dtype=torch.float64, device="cuda", generator=g)
+    r2 = torch.randn(no, no, nv, nv, dtype=torch.float64, device="cuda", generator=g)
+    want = r2 + 0.5 * torch.einsum("xa,xyzabc->yzbc", f, X.double())
+    _c_rccsdt.t3_r2_fock_(r2, X, f, no, nv, 0.5)
+    assert float((r2 - want).abs().max()) <= 1e-13 * float(want.abs().max())

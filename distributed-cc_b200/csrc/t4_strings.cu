@@ -197,9 +197,10 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// One run on warp tiles of 8 RT rows x 8 CT columns.  Fragments of m8n8k4: lane l holds
+// One run on warp tiles of 8 RT rows x 8 CT columns; AHEAD: with the loads of a step issued during
+// the products of the one before.  Fragments of m8n8k4: lane l holds
 // A[row l/4][k l%4], B[k l%4][col l/4] and D[row l/4][cols 2(l%4), 2(l%4)+1].
-template <int RT, int CT>
+template <bool AHEAD, int RT, int CT>
 __device__ __forceinline__ void t4s_run(double *acc, const T4Rec *rec, int r0, int r1, const T4Run &g,
                                         const int32_t *__restrict__ pair_sm, int nocc, int warp, int lane, int *status) {
     const int nrt = (g.R + 8 * RT - 1) / (8 * RT), nct = (g.C + 8 * CT - 1) / (8 * CT);
@@ -237,15 +238,15 @@ __device__ __forceinline__ void t4s_run(double *acc, const T4Rec *rec, int r0, i
                     k0 -= K0;
                     k1++;
                 }
-                for (int64_t kb = 0; kb < KK; kb += 4) {
-                    double a[RT], b[CT];
+                double a[RT], b[CT];
+                auto fetch = [&]() {  // this lane's elements of the step; zeros past the last summed value
                     if (k1 < K1) {
                         const double *Wk = W + (k0 * wk0 + k1 * wk1), *Tk = T + (k0 * tk0 + k1 * tk1);
 #pragma unroll
                         for (int u = 0; u < RT; ++u) a[u] = alpha * __ldg(Wk + wo[u]);
 #pragma unroll
                         for (int v = 0; v < CT; ++v) b[v] = __ldg(Tk + to[v]);
-                    } else {  // past the last summed value
+                    } else {
 #pragma unroll
                         for (int u = 0; u < RT; ++u) a[u] = 0.0;
 #pragma unroll
@@ -256,11 +257,31 @@ __device__ __forceinline__ void t4s_run(double *acc, const T4Rec *rec, int r0, i
                         k0 -= K0;
                         k1++;
                     }
-                    __syncwarp();
+                };
+                if constexpr (AHEAD) {
+                    fetch();
+                    for (int64_t kb = 0; kb < KK; kb += 4) {
+                        double x[RT], y[CT];
 #pragma unroll
-                    for (int u = 0; u < RT; ++u)
+                        for (int u = 0; u < RT; ++u) x[u] = a[u];
 #pragma unroll
-                        for (int v = 0; v < CT; ++v) dmma(d[u][v][0], d[u][v][1], a[u], b[v]);
+                        for (int v = 0; v < CT; ++v) y[v] = b[v];
+                        fetch();  // the next step's loads, in flight during this one's products
+                        __syncwarp();
+#pragma unroll
+                        for (int u = 0; u < RT; ++u)
+#pragma unroll
+                            for (int v = 0; v < CT; ++v) dmma(d[u][v][0], d[u][v][1], x[u], y[v]);
+                    }
+                } else {
+                    for (int64_t kb = 0; kb < KK; kb += 4) {
+                        fetch();
+                        __syncwarp();
+#pragma unroll
+                        for (int u = 0; u < RT; ++u)
+#pragma unroll
+                            for (int v = 0; v < CT; ++v) dmma(d[u][v][0], d[u][v][1], a[u], b[v]);
+                    }
                 }
             }
         }
@@ -325,6 +346,7 @@ __device__ __forceinline__ int t4s_cost(int R, int C, int RT, int CT) {
 }
 
 // Tile shapes of a run (8 RT rows x 8 CT columns per warp); -1: one row, on the FP64 lanes.
+template <bool AHEAD>
 __device__ void t4s_plan(T4Run &g, int rord, int cord, int na, int nv) {
     g.R = g.C = 1;
     for (int p = 0; p < 4; ++p) {
@@ -338,7 +360,9 @@ __device__ void t4s_plan(T4Run &g, int rord, int cord, int na, int nv) {
     }
     g.shape = -1;
     if (g.R == 1) return;
-    const int rt[8] = {4, 4, 3, 2, 8, 1, 8, 2}, ct[8] = {4, 3, 4, 8, 2, 8, 1, 2};
+    // at most 12 accumulators where a second set of operands is in flight
+    const int rt[8] = {AHEAD ? 2 : 4, 4, 3, 2, AHEAD ? 4 : 8, 1, 8, 2},
+              ct[8] = {AHEAD ? 6 : 4, 3, 4, AHEAD ? 4 : 8, 2, 8, 1, 2};
     int best = 0x7fffffff;
     for (int i = 0; i < 8; ++i) {  // the shape of least cost for these rows and columns
         const int c = t4s_cost(g.R, g.C, rt[i], ct[i]);
@@ -349,6 +373,11 @@ __device__ void t4s_plan(T4Run &g, int rord, int cord, int na, int nv) {
     }
 }
 
+// AHEAD where all CTAs are resident at once: a warp's loads then have little company to hide
+// behind, and issuing them a step ahead pays (nocc=4, nvir=12 0.80 -> 0.63 ms, nocc=6, nvir=9 1.08 ->
+// 0.93; nocc=5, nvir=8 the same 0.47); with more rounds the SMs are busy and the smaller tiles
+// cost more loads (nocc=7, nvir=11 3.56 -> 3.98).
+template <bool AHEAD>
 __global__ void __launch_bounds__(T4S_THREADS, 2)
     k_t4_strings(const __grid_constant__ T4StrOps ops, const int64_t *__restrict__ desc, int nstr,
                  const int32_t *__restrict__ quads, const int32_t *__restrict__ pair_off,
@@ -398,7 +427,7 @@ __global__ void __launch_bounds__(T4S_THREADS, 2)
             int e = i;
             bool any = false;
             for (; e < nb && same(i, e); e++) any = any || rec[e].ok;
-            if (any) t4s_plan(runs[i], rec[i].rord, rec[i].cord, na, nv);
+            if (any) t4s_plan<AHEAD>(runs[i], rec[i].rord, rec[i].cord, na, nv);
             runs[i].end = any ? e : -e;  // no string of the run passed its checks: skipped
         }
         __syncthreads();
@@ -411,14 +440,14 @@ __global__ void __launch_bounds__(T4S_THREADS, 2)
             }
 #define T4S_CASE(ID, RT, CT)                                                             \
     case ID:                                                                             \
-        t4s_run<RT, CT>(acc, rec, r0, r1, g, pair_sm, nocc, warp, lane, status);          \
+        t4s_run<AHEAD, RT, CT>(acc, rec, r0, r1, g, pair_sm, nocc, warp, lane, status);   \
         break;
             switch (g.shape) {
-                T4S_CASE(0, 4, 4)
+                T4S_CASE(0, (AHEAD ? 2 : 4), (AHEAD ? 6 : 4))
                 T4S_CASE(1, 4, 3)
                 T4S_CASE(2, 3, 4)
-                T4S_CASE(3, 2, 8)
-                T4S_CASE(4, 8, 2)
+                T4S_CASE(3, 2, (AHEAD ? 4 : 8))
+                T4S_CASE(4, (AHEAD ? 4 : 8), 2)
                 T4S_CASE(5, 1, 8)
                 T4S_CASE(6, 8, 1)
                 T4S_CASE(7, 2, 2)
@@ -554,11 +583,18 @@ extern "C" int dcc_t4_strings(const double *const *ops, const int64_t *op_numel,
     DCC_REQUIRE(grid < (1LL << 31), DCC_ERR_SHAPE, "too many blocks");
     const size_t smem = (size_t)na * nvir * nvir * nvir * sizeof(double) + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run));
     static_assert(T4S_SMEM_MAX + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run)) <= 227 * 1024, "shared memory per CTA");
-    cudaFuncSetAttribute(k_t4_strings, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(T4S_SMEM_MAX + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run))));
-    k_t4_strings<<<(unsigned)grid, T4S_THREADS, smem, as_stream(stream)>>>(
-        o, desc, nstr, quads, pair_off, pair_sm, ngroups, (int)npairs, (int)nocc, (int)nvir, na, nsplit, beta, r4,
-        status);
+    const int64_t slots = 148 * (2 * ((int64_t)smem + 1024) <= 228 * 1024 ? 2 : 1);
+    auto launch = [&](auto kern) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(T4S_SMEM_MAX + T4S_BATCH * (sizeof(T4Rec) + sizeof(T4Run))));
+        kern<<<(unsigned)grid, T4S_THREADS, smem, as_stream(stream)>>>(o, desc, nstr, quads, pair_off, pair_sm, ngroups,
+                                                                       (int)npairs, (int)nocc, (int)nvir, na, nsplit,
+                                                                       beta, r4, status);
+    };
+    if (grid <= slots)
+        launch(k_t4_strings<true>);
+    else
+        launch(k_t4_strings<false>);
     return launch_status("t4_strings");
 }
 

@@ -76,8 +76,8 @@ class T4Iteration:
 
 
 class T4IterationGraph:
-    """T4Iteration captured as one CUDA graph: the ~300 small launches of the T4
-    residual at nvir ~ 11 (einsums, block forms, scatters) replay without per-launch host
+    """T4Iteration captured as one CUDA graph: the some 140 launches of the T4
+    residual at nvir ~ 11 (mostly the builders' einsums) replay without per-launch host
     overhead.  New inputs are copied into the same tensors before `replay()`."""
 
     def __init__(self, it):

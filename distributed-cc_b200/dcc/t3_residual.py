@@ -33,9 +33,10 @@ T2 and T5/2 as one GEMM over the concatenated contraction index; T1 reusing
 T2's U operand; the K = nocc^2 W_oooo / F_oo part over a K-major split of U),
 and one gather kernel applies the symmetrization to S (the FP64 path builds S
 the same way from DGEMMs, one occupied slice at a time).  W_vvvv.t3 (three strings, the dominant cost) are
-three split-precision GEMMs that accumulate straight into r3; the three
-F_vv.t3 strings ride in them as extra terms of the W operand
-(contract.WvvvvT3).  The FP64 path runs F_vv.t3 as batched DGEMMs.
+split-precision GEMMs: over symmetric and antisymmetric index pairs where W_vvvv has the pair
+symmetry and nvir >= 60 (contract.PairWvvvvT3: half the products, one pass adds the results to
+r3), else three that accumulate straight into r3; the three F_vv.t3 strings ride in either as
+extra terms of the W operand.  The FP64 path runs F_vv.t3 as batched DGEMMs.
 
 precision = "fp64" runs every contraction in FP64 (cuBLAS DGEMM through
 torch): the plain FP64 GPU path.  "bf16x3" / "tf32x3" run the large

@@ -521,8 +521,9 @@ def compute_r4_tri_(r4, eris, F_vv, W_vvvo, W_vooo, W_vvvv, W_oooo, W_ovov, t2, 
     launch of the fused strings kernel (dcc_t4_strings: a CTA per stored block and row range
     holds its r4 rows in shared memory and runs every string over them, operands read in
     place through the descriptors of fused_plan), and with F_oo given the OO batch joins
-    the same launch (its F_oo / W_oooo slots as strings over the unpacked T4, its W_ovov /
-    W_voov strings in pair mode over the sparse (source, output) pair lists).  Their
+    the same launch, as strings over T4 unpacked to every ordering (and P4_201 of it; with the
+    caller's `forms` its W_ovov / W_voov strings run in pair mode over the sparse (source, output)
+    pair lists instead).  Their
     contractions are short (K = nvir, nocc, nocc^2 or nocc nvir), so they are FP64 in every
     precision; in FP64 the F_vv / W_vvvv strings join the same launch, and precision
     "bf16x3"/"tf32x3" runs those (K = nvir^2) as split GEMMs.  The builders stay FP64.  On the CPU (the formulation

@@ -24,7 +24,7 @@
 // What bounds it: operand loads (L1) and the FP64 matrix pipe; the contractions are short
 // (7 to 121 summed values).  Measured (nocc=7, nvir=11, 161 blocks, B200): the kernel 3.5 ms, against
 // 8.3 ms with FP64 lanes, one barrier and one shared-memory update per string and pair; at
-// nocc=5, nvir=8 0.45 against 2.2 ms.
+// nocc=5, nvir=8 0.47 against 2.2 ms.
 //
 // The W_ovov / W_voov strings of the OO batch (distr_cc/rccsdtq.py:1062-1349) take a
 // stored SOURCE block and an occupied m per term: they run in "pair mode", once for

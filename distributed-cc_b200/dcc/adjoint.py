@@ -130,9 +130,16 @@ def vjp(lam, t2, t3, F_vv, F_oo, W_vvvo, W_vooo, W_vvvv, W_ovov, W_ovvo, Ws, pre
     E('ijkabc,lbid->jkldca', Lam, W_ovov, gU, -1.0, 0.0)
     E('ijkabc,laid->jkldcb', Lam, G2, gU)
     E('ijkabc,ladi->jklbcd', Lam, W_ovvo, gU, 0.5)
-    # Ws and F_oo together: F_oo[l,i] at m = j (its own GEMM had nocc columns of a 256-column tile)
-    eye = torch.eye(nocc, dtype=f64, device=dev)
-    E('ijkabc,lmij->lmkabc', Lam, (Ws - F_oo[:, None, :, None] * eye[None, :, None, :]).contiguous(), gU, 0.5)
+    # FP64: Ws and F_oo together, F_oo[l,i] at m = j.  A split product keeps F apart here and below:
+    # the sum runs in FP32, and F, the larger part, would be rounded once per term of W's longer sum.
+    # gt3's error against FP64, joined / apart: bf16x3 at nocc=6, nvir=40 4.5e-6 / 3.5e-6 (forward and
+    # backward 6.4 / 8.2 ms), tf32x3 there 6.6e-6 / 3.3e-6, at nocc=4, nvir=12 6.3e-7 / 1.9e-7.
+    if kind is None:
+        eye = torch.eye(nocc, dtype=f64, device=dev)
+        E('ijkabc,lmij->lmkabc', Lam, (Ws - F_oo[:, None, :, None] * eye[None, :, None, :]).contiguous(), gU, 0.5)
+    else:
+        E('ijkabc,lmij->lmkabc', Lam, Ws, gU, 0.5)
+        E('ijkabc,li->ljkabc', Lam, F_oo, gU, -0.5)
     del Lam
     # unpack^T then the projection: (1/|stab|) * sum over all six permutations
     gt3 = torch.empty_like(t3)
@@ -149,16 +156,19 @@ def vjp(lam, t2, t3, F_vv, F_oo, W_vvvo, W_vooo, W_vvvv, W_ovov, W_ovvo, Ws, pre
     E('qabc,qadc->bd', lam, t3, gFvv)
     E('qabc,qabd->cd', lam, t3, gFvv)
     gd = torch.empty_like(t3)
-    # F_vv rides in the W operands, as in the forward (contract.WvvvvT3)
-    W1 = W_vvvv.clone()
-    W1.diagonal(0, 1, 3).add_(F_vv.unsqueeze(2))  # F[a,d] delta(b,e)
-    W1.diagonal(0, 0, 2).add_(F_vv.unsqueeze(2))  # delta(a,d) F[b,e]
+    W1 = W3 = W_vvvv
+    if kind is None:  # F_vv rides in the W operands
+        W1, W3 = W_vvvv.clone(), W_vvvv.clone()
+        W1.diagonal(0, 1, 3).add_(F_vv.unsqueeze(2))  # F[a,d] delta(b,e)
+        W1.diagonal(0, 0, 2).add_(F_vv.unsqueeze(2))  # delta(a,d) F[b,e]
+        W3.diagonal(0, 0, 2).add_(F_vv.unsqueeze(2))  # delta(b,d) F[c,e]
     E('qabc,abde->qdec', lam, W1, gd, 1.0, 0.0)
     E('qabc,acde->qdbe', lam, W_vvvv, gd)
-    W1.copy_(W_vvvv)
-    W1.diagonal(0, 0, 2).add_(F_vv.unsqueeze(2))  # delta(b,d) F[c,e]
-    E('qabc,bcde->qade', lam, W1, gd)
-    del W1
+    E('qabc,bcde->qade', lam, W3, gd)
+    if kind is not None:
+        E('qabc,ad->qdbc', lam, F_vv, gd)
+        E('qabc,bd->qadc', lam, F_vv, gd)
+        E('qabc,cd->qabd', lam, F_vv, gd)
     gt3.add_(stab_project(gd, ijk))
     return gt2, gt3, gFvv, gFoo, gWvvvo, gWvooo, gWvvvv, gWovov, gWovvo, gWoooo
 

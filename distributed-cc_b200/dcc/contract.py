@@ -374,16 +374,33 @@ L.bind("dcc_gemm_grouped_table_bytes", [L.c_int], L.c_size)
 SPLIT_SPEC, GEMM_SPEC = 22, 25
 
 
+def check_grouped_spans(spec, numel):
+    """The maps of every operand of a grouped split stay inside its source of numel[p] elements (what
+    _check_span asks of a single split's tensor)."""
+    if len(numel) != len(spec):
+        raise ValueError("need the elements of %d sources" % len(spec))
+    for p, (row, n) in enumerate(zip(spec, numel)):
+        M, K, fm, fk = int(row[2]), int(row[3]), [int(x) for x in row[7:14]], [int(x) for x in row[14:21]]
+        if any(x < 0 for x in fm[3:] + fk[3:]):
+            raise ValueError("operand %d: negative map strides" % p)
+        if M > 0 and K > 0 and _max_offset(fm, M) + _max_offset(fk, K) >= n:
+            raise ValueError("operand %d: the address maps reach past its source" % p)
+
+
 class GroupedSplit:
     """Operand splits of many einsums in one launch (dcc_split_grouped).
 
     spec: int64 [n, 22] rows (hi, lo, M, K, kw, ld, k0, row map(7), k map(7),
-    source is float32); run(srcs) fills every operand from its source address."""
+    source is float32); run(srcs) fills every operand from its source address.
+    numel: the elements each source has from its address on, against which the maps are
+    checked here (run sees addresses alone)."""
 
-    def __init__(self, spec, kind, device):
+    def __init__(self, spec, kind, device, numel=None):
         spec = np.ascontiguousarray(spec, dtype=np.int64)
         if spec.ndim != 2 or spec.shape[1] != SPLIT_SPEC:
             raise ValueError("spec must be int64 [n, %d]" % SPLIT_SPEC)
+        if numel is not None:
+            check_grouped_spans(spec, numel)
         self.n, self.kind = spec.shape[0], int(kind)
         nbytes = int(L.lib().dcc_split_grouped_table_bytes(self.n))
         self.table = torch.empty(nbytes, dtype=torch.uint8, device=device)

@@ -281,21 +281,30 @@ class T3Residual:
             self._small = self._small_split()
 
     # ------------------------------------------------------------ pieces
-    def _small_split(self):
-        """One grouped split for the operands of the S GEMMs made from t2 and the W intermediates
-        (seven launches of a few us of work each otherwise), in the order _s_split lists them."""
+    def _small_ops(self):
+        """(operand, piece, row map, k map, elements of the source) of the S GEMMs' operands made from t2
+        and the W intermediates, in the order of _fill_small's sources."""
         no, nv, c, pl = self.no, self.nv, contract, self.plan
-        ops = [(self.ya, 0, c.three(nv, no, no, 1, no ** 3), c.lin(no * no)),
-               (self.yb, 0, c.lin(1), c.lin(no * nv * nv)),
-               (self.xa, 0) + pl["x"]["a"][0][1:], (self.xb, 0) + pl["x"]["b"][0][1:]]
+        ov2 = (no * nv) ** 2
+        # -Y: rows (i,j,a) of W_vooo[a,l,i,j] and columns (k,b,c) of t2[l,k,b,c], K = l
+        ops = [(self.ya, 0, c.three(no, nv, no, 1, no ** 3), c.lin(no * no), nv * no ** 3),
+               (self.yb, 0, c.lin(1), c.lin(no * nv * nv), ov2),
+               (self.xa, 0) + pl["x"]["a"][0][1:] + (nv ** 3 * no,), (self.xb, 0) + pl["x"]["b"][0][1:] + (ov2,)]
         if self.with_oo:
-            ops += [(self.ooa, i) + pl["oo"]["a"][i][1:] for i in range(2)] + [(self.t1a, 0) + pl["t1"]["a"][0][1:]]
-        spec = []
-        for op, i, fm, fk in ops:
+            ops += [(self.ooa, i) + pl["oo"]["a"][i][1:] + (ov2,) for i in range(2)]
+            ops += [(self.t1a, 0) + pl["t1"]["a"][0][1:] + (ov2,)]
+        return ops
+
+    def _small_split(self):
+        """One grouped split for the operands of _small_ops (seven launches of a few us of work each
+        otherwise)."""
+        c, spec, numel = contract, [], []
+        for op, i, fm, fk, n in self._small_ops():
             off, k, w = op.pieces[i]
             spec.append([op.hi.data_ptr(), op.lo.data_ptr(), op.M, k, w, op.Kp, off] + list(c.as4(fm)) + list(c.as4(fk))
                         + [0])
-        return c.GroupedSplit(spec, self.kind, self.dev)
+            numel.append(n)
+        return c.GroupedSplit(spec, self.kind, self.dev, numel)
 
     def _oo_sources(self, d):
         """{G2, Wvo_half, W_ovov} of the OO GEMMs and, on a CUDA device with d's tensors laid out
@@ -326,28 +335,19 @@ class T3Residual:
         return woooo_foo_matrix(d.W_oooo, d.F_oo, SYM_TOL, assume_symmetric=self.woooo_pair_symmetric)
 
     def _fill_small(self, d):
-        """The operands of _small_split from d's tensors; returns the OO sources it made."""
-        no, nv = self.no, self.nv
-        src = {}
-        srcs = [(d.W_vooo, nv * no ** 3), (d.t2, (no * nv) ** 2), (d.W_vvvo, nv ** 3 * no), (d.t2, (no * nv) ** 2)]
+        """The operands of _small_ops from d's tensors."""
+        srcs = [d.W_vooo, d.t2, d.W_vvvo, d.t2]
         if self.with_oo:
             src = self._oo_sources(d)
-            srcs += [(src[n], (no * nv) ** 2) for n in ("G2", "Wvo_half", "W_ovov")]
+            srcs += [src[n] for n in ("G2", "Wvo_half", "W_ovov")]
+        ops = self._small_ops()
         if self._small is not None and all(t.dtype == f64 and t.is_cuda and t.is_contiguous() and t.numel() == n
-                                           for t, n in srcs):
-            self._small.run([t.data_ptr() for t, _ in srcs])
+                                           for t, (_, _, _, _, n) in zip(srcs, ops)):
+            self._small.run([t.data_ptr() for t in srcs])
             return
         # other layouts and types: one by one, each through its own checks
-        c, pl = contract, self.plan
-        self.ya.fill(d.W_vooo, c.three(nv, no, no, 1, no ** 3), c.lin(no * no))
-        self.yb.fill(d.t2, c.lin(1), c.lin(no * nv * nv))
-        self.xa.fill(d.W_vvvo, *pl["x"]["a"][0][1:])
-        self.xb.fill(d.t2, *pl["x"]["b"][0][1:])
-        if self.with_oo:
-            for i, (name, fm, fk) in enumerate(pl["oo"]["a"]):
-                self.ooa.fill_piece(i, src[name], fm, fk)
-            name, fm, fk = pl["t1"]["a"][0]
-            self.t1a.fill(src[name], fm, fk)
+        for t, (op, i, fm, fk, _) in zip(srcs, ops):
+            op.fill_piece(i, t, fm, fk)
 
     def _gemm(self, name, A, B, C, frow, fcol, alpha, beta, Kp=None):
         """One of the S GEMMs under the tile and raster configuration tuned for it (tune()); its
@@ -360,13 +360,11 @@ class T3Residual:
     def _gkey(self, name):
         return ("s_gemm", name, self.no, self.nv, self.kind)
 
-    def _y_into_s(self, d):
+    def _y_into_s(self):
         """S = -Y in S's [i][j][k][a][b][c] layout (split path): rows (i,j,a), columns (k,b,c).  Y
         then rides in S's permutation sum, and the gather reads one source instead of two."""
         no, nv = self.no, self.nv
         c = contract
-        self.ya.fill(d.W_vooo, c.three(no, nv, no, 1, no ** 3), c.lin(no * no))
-        self.yb.fill(d.t2, c.lin(1), c.lin(no * nv * nv))
         self._gemm("y", self.ya, self.yb, self.S, c.three(no, nv, no * no * nv ** 3, no * nv ** 3, nv * nv),
                    c.two(nv * nv, nv ** 3, 1), -1.0, 0.0)
 
@@ -430,7 +428,7 @@ class T3Residual:
         S = self.S
         x = pl["x"]
         self._fill_small(d)
-        self._y_into_s(d)  # writes S first
+        self._y_into_s()  # writes S first
         self._gemm("x", self.xa, self.xb, S, *x["out"], x["alpha"], 1.0)
         if not self.with_oo:
             return

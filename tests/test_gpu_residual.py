@@ -256,3 +256,31 @@ def test_oo_operands(no, nv):
         want, wa = t.woooo_foo_matrix(d.W_oooo, d.F_oo)
         assert torch.equal(A, want) and (Wa is None) == (wa is None)
         assert (Wa is None) == (case == "symmetric" or no == 1)
+
+
+@pytest.mark.parametrize("no,nv", [(5, 3), (9, 2), (10, 7), (4, 9)])
+@pytest.mark.parametrize("precision", ["bf16x3", "tf32x3"])
+def test_small_operands(mods, precision, no, nv):
+    """The S operands split in one grouped launch hold the pieces of single splits of the permuted
+    sources, bit for bit, and are the ones the residual uses: the split step against the FP64
+    path, with fewer virtual than occupied indices too."""
+    syn, tr, _ = mods
+    from dcc import contract as c
+    d = syn.make_inputs(no, nv, seed=no)
+    res = tr.T3Residual(no, nv, precision, with_oo=True)
+    got = res.compute(d, d.t3)
+    assert res.status_ok()
+    G2 = -0.5 * (d.W_ovov + d.W_ovvo.permute(0, 1, 3, 2))
+    want = [(res.ya, 0, d.W_vooo.permute(2, 3, 0, 1).reshape(-1, no)),  # (i,j,a), l
+            (res.yb, 0, d.t2.permute(1, 2, 3, 0).reshape(-1, no)),  # (k,b,c), l
+            (res.xa, 0, d.W_vvvo.permute(3, 0, 1, 2).reshape(-1, nv)),  # (j,a,b), d
+            (res.xb, 0, d.t2.permute(0, 1, 3, 2).reshape(-1, nv)),  # (i,k,c), d
+            (res.ooa, 0, G2.permute(2, 1, 0, 3).reshape(no * nv, -1)),  # (i,a), (l,d)
+            (res.ooa, 1, 0.5 * d.W_ovvo.permute(3, 1, 0, 2).reshape(no * nv, -1)),
+            (res.t1a, 0, d.W_ovov.permute(2, 1, 0, 3).reshape(no * nv, -1))]  # (i,b), (l,d)
+    for op, i, x in want:
+        off, k, _ = op.pieces[i]
+        one = c.Split(x.shape[0], k, op.kind).fill(x.contiguous(), c.lin(k), c.lin(1))
+        assert torch.equal(op.hi[:, off:off + k], one.hi[:, :k]) and torch.equal(op.lo[:, off:off + k], one.lo[:, :k])
+    ref = tr.T3Residual(no, nv, "fp64", with_oo=True).compute(d, d.t3)
+    assert float((got - ref).abs().max() / ref.abs().max()) < TOL[precision]

@@ -3,6 +3,7 @@ dcc_gemm_split3, checked on the CPU: the split, the GEMM and the epilogue
 scatter are emulated in numpy with the same three-digit map arithmetic the
 kernels use, and compared with numpy einsums of the terms they implement."""
 import numpy as np
+import pytest
 
 from dcc import contract as c
 
@@ -144,3 +145,48 @@ def test_einsum_into_maps():
         gemm(A, B, base.numpy(), c._map_of(gM, 1), c._map_of(gN, 1), 1.0, 0.0)
         np.testing.assert_allclose(out.numpy(), ref.numpy(), rtol=0, atol=1e-12)
     assert checked >= 4
+
+
+def _small_operands(monkeypatch, no, nv):
+    """(T3Residual, the rows of the grouped split of its S operands), on the CPU."""
+    from dcc import t3_residual as tr
+    res = tr.T3Residual(no, nv, "bf16x3", device="cpu")
+    spec = []
+    monkeypatch.setattr(c, "GroupedSplit", lambda rows, *a, **k: spec.extend(rows))
+    res._small_split()
+    return res, spec
+
+
+@pytest.mark.parametrize("no,nv", [(3, 4), (4, 4), (5, 3), (9, 2), (10, 7), (2, 1)])
+def test_small_operand_maps(monkeypatch, no, nv):
+    """The grouped split of the S operands made from t2 and the W intermediates reads inside every
+    source (nvir below nocc too, where swapped radices reach past W_vooo), and its rows are the
+    operands of -Y: W_vooo[a,l,i,j] as rows (i,j,a) and t2[l,k,b,c] as rows (k,b,c), over l."""
+    res, spec = _small_operands(monkeypatch, no, nv)
+    rng = np.random.default_rng(no)
+    Wvooo, t2 = rng.standard_normal((nv, no, no, no)), rng.standard_normal((no, no, nv, nv))
+    numel = [Wvooo.size, t2.size, nv ** 3 * no, t2.size] + [(no * nv) ** 2] * 3
+    assert len(spec) == len(numel)
+    for row, n in zip(spec, numel):
+        M, K, fm, fk = row[2], row[3], row[7:14], row[14:21]
+        assert int(fmap(fm, np.arange(M)).max() + fmap(fk, np.arange(K)).max()) == n - 1  # all of it, no more
+    M, K, fm, fk = spec[0][2], spec[0][3], spec[0][7:14], spec[0][14:21]
+    assert spec[0][0] == res.ya.hi.data_ptr() and spec[1][0] == res.yb.hi.data_ptr()
+    np.testing.assert_array_equal(split(Wvooo, M, K, fm, fk), Wvooo.transpose(2, 3, 0, 1).reshape(-1, no))
+    M, K, fm, fk = spec[1][2], spec[1][3], spec[1][7:14], spec[1][14:21]
+    np.testing.assert_array_equal(split(t2, M, K, fm, fk), t2.transpose(1, 2, 3, 0).reshape(-1, no))
+
+
+def test_grouped_split_refuses_a_map_past_its_source():
+    """A grouped operand whose map reaches past its source's elements is refused on the host, as a
+    single split refuses it."""
+    row = [0, 0, 6, 4, 64, 64, 0] + list(c.as4(c.lin(4))) + list(c.as4(c.lin(1))) + [0]
+    c.check_grouped_spans([row], [24])
+    for bad in ([23], [0]):
+        with pytest.raises(ValueError):
+            c.check_grouped_spans([row], bad)
+    with pytest.raises(ValueError):
+        c.check_grouped_spans([row[:7] + list(c.as4(c.lin(-1))) + row[14:]], [24])
+    c.check_grouped_spans([row[:3] + [0] + row[4:]], [0])  # nothing to read
+    with pytest.raises(ValueError):
+        c.check_grouped_spans([row], [24, 24])

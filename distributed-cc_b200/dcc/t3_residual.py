@@ -345,9 +345,10 @@ class T3Residual:
                                            for t, (_, _, _, _, n) in zip(srcs, ops)):
             self._small.run([t.data_ptr() for t in srcs])
             return
-        # other layouts and types: one by one, each through its own checks
+        # other layouts and types: one by one, each through its own checks (the maps are those of a
+        # contiguous source)
         for t, (op, i, fm, fk, _) in zip(srcs, ops):
-            op.fill_piece(i, t, fm, fk)
+            op.fill_piece(i, t.contiguous(), fm, fk)
 
     def _gemm(self, name, A, B, C, frow, fcol, alpha, beta, Kp=None):
         """One of the S GEMMs under the tile and raster configuration tuned for it (tune()); its

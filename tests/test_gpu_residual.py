@@ -284,3 +284,18 @@ def test_small_operands(mods, precision, no, nv):
         assert torch.equal(op.hi[:, off:off + k], one.hi[:, :k]) and torch.equal(op.lo[:, off:off + k], one.lo[:, :k])
     ref = tr.T3Residual(no, nv, "fp64", with_oo=True).compute(d, d.t3)
     assert float((got - ref).abs().max() / ref.abs().max()) < TOL[precision]
+
+
+@pytest.mark.parametrize("with_oo", [False, True])
+def test_strided_inputs(mods, with_oo):
+    """Intermediates and t2 laid out in memory in another order give the residual of contiguous ones
+    (bit for bit: the same operands)."""
+    syn, tr, _ = mods
+    no, nv = 9, 4
+    d = syn.make_inputs(no, nv, seed=5)
+    res = tr.T3Residual(no, nv, "bf16x3", with_oo=with_oo)
+    want = res.compute(d, d.t3).clone()
+    for n in ("t2", "W_vooo", "W_vvvo", "W_ovov", "W_ovvo", "W_oooo", "W_vvvv"):
+        setattr(d, n, getattr(d, n).permute(3, 1, 0, 2).contiguous().permute(2, 1, 3, 0))
+        assert torch.equal(res.compute(d, d.t3), want), n
+    assert res.status_ok()

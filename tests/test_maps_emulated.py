@@ -190,3 +190,36 @@ def test_grouped_split_refuses_a_map_past_its_source():
     c.check_grouped_spans([row[:3] + [0] + row[4:]], [0])  # nothing to read
     with pytest.raises(ValueError):
         c.check_grouped_spans([row], [24, 24])
+
+
+def test_small_operands_of_strided_sources(monkeypatch):
+    """Sources in another memory order than the maps' are split by their values, not by their place in
+    memory: every operand from strided views equals the one from contiguous tensors."""
+    import torch
+    from dcc import t3_residual as tr
+    no, nv = 3, 4
+    rng = np.random.default_rng(7)
+    shapes = {"W_vooo": (nv, no, no, no), "t2": (no, no, nv, nv), "W_vvvo": (nv, nv, nv, no), "W_ovov": (no, nv, no, nv),
+              "W_ovvo": (no, nv, nv, no), "W_oooo": (no,) * 4, "F_oo": (no, no)}
+    plain = {k: torch.from_numpy(rng.standard_normal(s)) for k, s in shapes.items()}
+    got = []
+
+    def fill_piece(self, i, src, fm, fk):
+        k = self.pieces[i][1]
+        flat = src.as_strided((src.untyped_storage().size() // 8 - src.storage_offset(),), (1,)).numpy()
+        got.append(split(flat, self.M, k, fm, fk))
+
+    monkeypatch.setattr(c.Split, "fill_piece", fill_piece)
+    res = tr.T3Residual(no, nv, "bf16x3", device="cpu")
+    for order in (None, (3, 2, 1, 0), (1, 0, 3, 2)):
+        class D:
+            pass
+        for k, t in plain.items():
+            if order is not None and t.dim() == 4:  # the same values, laid out in memory by `order`
+                t = t.permute(order).contiguous().permute([order.index(x) for x in range(4)])
+            setattr(D, k, t)
+        res._fill_small(D)
+    assert len(got) == 21
+    for a, b, x in zip(got[:7], got[7:14], got[14:]):
+        np.testing.assert_array_equal(a, b)
+        np.testing.assert_array_equal(a, x)

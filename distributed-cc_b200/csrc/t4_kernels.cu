@@ -133,11 +133,22 @@ __global__ void k_unpack_t4(const double *src, double *out, int64_t loc, int ax0
 // otherwise.  Bound by the writes (16 bytes per element of the ordered space, 0.09 ms at 6.5 TB/s at
 // nocc=7, nvir=11) and the latency of one staged block per SM: 0.235 ms there, against 2.0 ms for a
 // gather and a scatter per axis permutation, a copy and the orbit kernel (50 launches).
+//
+// The digits of an element come from a multiplied reciprocal (Granlund and Montgomery, 1994): with
+// 2^(l-1) < nv <= 2^l and m = ceil(2^(31+l) / nv), which fits 32 bits, x / nv = (x m) >> (31 + l) for
+// every x < 2^31, since x (m nv - 2^(31+l)) < 2^31 2^l.  nv^4 < 2^31 wherever nv < 128.
 struct T4Magic {
-    uint32_t m;  // ceil(2^32 / nv): x / nv = (x m) >> 32 for x < 2^32 / nv
-    int nv;
-    __device__ __forceinline__ int div(int x) const { return (int)__umulhi((uint32_t)x, m); }
+    uint32_t m;
+    int sh, nv;  // sh: l - 1
+    __device__ __forceinline__ int div(int x) const { return (int)(__umulhi((uint32_t)x, m) >> sh); }
 };
+static T4Magic t4_magic(int nv) {
+    int l = 1;
+    while ((1 << l) < nv) l++;
+    // nv = 1 divides x = 0 alone
+    const uint32_t m = nv == 1 ? 0u : (uint32_t)(((1ull << (31 + l)) + (uint64_t)nv - 1) / (uint64_t)nv);
+    return T4Magic{m, l - 1, nv};
+}
 
 template <bool SMEM>
 __global__ void __launch_bounds__(512) k_t4_unpack_all(const double *__restrict__ t4, const int32_t *__restrict__ src,
@@ -275,7 +286,7 @@ extern "C" int dcc_t4_unpack_all(const double *t4, const int32_t *src, const int
     DCC_REQUIRE(norder >= 0 && norder < (1LL << 31) && nvir >= 0 && nvir < 128, DCC_ERR_SHAPE, "bad size");
     if (norder == 0 || nvir == 0) return DCC_OK;
     DCC_REQUIRE(t4 && src && rank && T && Ts, DCC_ERR_NULL, "NULL buffer");
-    const T4Magic mg = {(uint32_t)(((1ull << 32) + (uint64_t)nvir - 1) / (uint64_t)nvir), (int)nvir};
+    const T4Magic mg = t4_magic((int)nvir);
     const int pitch = (int)(nvir | 1);
     const size_t smem = (size_t)pitch * pitch * pitch * pitch * sizeof(double);
     const int threads = nvir >= 9 ? 512 : 256;

@@ -546,7 +546,7 @@ def compute_r4_tri_(r4, eris, F_vv, W_vvvo, W_vooo, W_vvvv, W_oooo, W_ovov, t2, 
         # F_oo is given; the W_vvvv strings join it in FP64 and run as split GEMMs otherwise
         dense = kind is None
         oo = False if F_oo is None else ("full" if forms is None else True)
-        if own_spin4 and nv < 128:
+        if own_spin4:
             T4full, T4s = (x.view((nocc,) * 4 + (nv,) * 4) for x in _c_rccsdtq.t4_unpack_all(
                 t4.contiguous(), *_unpack_table(nocc, t4.device), nocc, nv))
         else:

@@ -262,3 +262,23 @@ def test_t4_feedback(oracle, precision, no, nv):
     tol = 1e-11 if precision == "fp64" else 1e-4
     assert np.abs(got2 - want2).max() <= tol * np.abs(want2 - r2).max()
     assert np.abs(got3 - want3).max() <= tol * np.abs(want3 - r3).max()
+
+
+@pytest.mark.parametrize("nv", [2, 64, 84, 85, 93, 127])
+def test_unpack_all_large_blocks(nv):
+    """t4_unpack_all up to the largest nvir it takes, on one ordering whose axes are permuted: every
+    element's digits are right (a reciprocal that is exact below 2^32 / nvir alone goes wrong
+    from nvir = 85 on).  == : the same products and sums."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from dcc import _c_rccsdtq
+    t4 = torch.randn((1,) + (nv,) * 4, dtype=torch.float64, device="cuda",
+                     generator=torch.Generator(device="cuda").manual_seed(nv))
+    axes = (3, 0, 2, 1)  # axis m of the ordering is axis axes[m] of the stored block
+    rank = torch.tensor([sum(a << (4 * m) for m, a in enumerate(axes))], dtype=torch.int32, device="cuda")
+    src = torch.zeros(1, dtype=torch.int32, device="cuda")
+    T, Ts = _c_rccsdtq.t4_unpack_all(t4, src, rank, 1, nv)
+    want = t4[0].permute(axes)
+    assert torch.equal(T[0], want)
+    want = 2.0 * want - want.transpose(0, 1) - want.transpose(0, 2) - want.transpose(0, 3)
+    assert torch.equal(Ts[0], want)

@@ -476,12 +476,13 @@ class T3Residual:
         r3.view(n * nv * nv, nv).add_(torch.matmul(t3.view(n * nv * nv, nv), F.t()))
         return r3
 
-    def wvvvv_(self, r3, d, t3):
-        """W_vvvv.t3 (distr_cc/rccsdt.py:421-427); in split precision F_vv.t3 rides in the same GEMMs."""
+    def wvvvv_(self, r3, d, t3, scratch=None):
+        """W_vvvv.t3 (distr_cc/rccsdt.py:421-427); in split precision F_vv.t3 rides in the same GEMMs.
+        scratch: a tensor that may be overwritten (the pair form's results; a buffer of its own
+        otherwise)."""
         if self.precision == "fp64":
             return contract.wvvvv_t3_fp64_(r3, d.W_vvvv, t3)
-        # S has been gathered: its buffer holds the pair results
-        if self.pairs is not None and self.pairs(r3, d.W_vvvv, t3, F=d.F_vv, scratch=self.S):
+        if self.pairs is not None and self.pairs(r3, d.W_vvvv, t3, F=d.F_vv, scratch=scratch):
             return r3
         return self.wvvvv(r3, d.W_vvvv, t3, F=d.F_vv)
 
@@ -537,7 +538,7 @@ class T3Residual:
             torch.cuda.current_stream().wait_event(wvvvv_ready)
         if self.precision == "fp64":
             self.fvv_(r3, d, t3)
-        self.wvvvv_(r3, d, t3)
+        self.wvvvv_(r3, d, t3, scratch=S)  # S has been gathered
         return r3
 
     def status_ok(self):

@@ -299,3 +299,21 @@ def test_strided_inputs(mods, with_oo):
         setattr(d, n, getattr(d, n).permute(3, 1, 0, 2).contiguous().permute(2, 1, 3, 0))
         assert torch.equal(res.compute(d, d.t3), want), n
     assert res.status_ok()
+
+
+def test_wvvvv_leaves_s_alone(mods):
+    """W_vvvv.t3 called by itself between s_ and the gather: S keeps its values (nvir = 60 takes the
+    pair form, whose results compute() alone may put into S)."""
+    syn, tr, _ = mods
+    no, nv = 2, 60
+    d = syn.make_inputs(no, nv, seed=6)
+    res = tr.T3Residual(no, nv, "bf16x3")
+    want = res.compute(d, d.t3).clone()
+    S = res.s_(d, d.t3)
+    keep = S.clone()
+    r3 = res.wvvvv_(torch.zeros_like(d.t3), d, d.t3)
+    assert res.pairs is not None and torch.equal(S, keep)
+    g = torch.empty_like(r3)
+    tr.s3_gather_f32_(g, d.ijk, nv, 0.0, S, 1.0, no)
+    # the two parts added here, in one rounding more or less of FP64 than compute() adds them
+    assert float((g + r3 - want).abs().max()) <= 1e-14 * float(g.abs().max() + r3.abs().max())

@@ -482,7 +482,9 @@ class T3Residual:
         otherwise)."""
         if self.precision == "fp64":
             return contract.wvvvv_t3_fp64_(r3, d.W_vvvv, t3)
-        if self.pairs is not None and self.pairs(r3, d.W_vvvv, t3, F=d.F_vv, scratch=scratch):
+        # the pair form reads W_vvvv's symmetry back to the host, which a stream under capture cannot
+        if self.pairs is not None and not torch.cuda.is_current_stream_capturing() and self.pairs(
+                r3, d.W_vvvv, t3, F=d.F_vv, scratch=scratch):
             return r3
         return self.wvvvv(r3, d.W_vvvv, t3, F=d.F_vv)
 

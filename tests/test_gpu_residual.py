@@ -317,3 +317,31 @@ def test_wvvvv_leaves_s_alone(mods):
     tr.s3_gather_f32_(g, d.ijk, nv, 0.0, S, 1.0, no)
     # the two parts added here, in one rounding more or less of FP64 than compute() adds them
     assert float((g + r3 - want).abs().max()) <= 1e-14 * float(g.abs().max() + r3.abs().max())
+
+
+def test_capture_without_oo_terms(mods):
+    """compute() without the OO terms reads nothing back to the host under graph capture, also where
+    the pair form of W_vvvv.t3 would run (nvir >= 60): the replay equals the plain form bit for bit."""
+    syn, tr, _ = mods
+    no, nv = 2, 60
+    d = syn.make_inputs(no, nv, seed=8)
+    plain = tr.T3Residual(no, nv, "bf16x3", with_oo=False, woooo_pair_symmetric=True)  # keeps the plain form
+    want = plain.compute(d, d.t3).clone()
+    res = tr.T3Residual(no, nv, "bf16x3", with_oo=False)
+    assert plain.pairs is None and res.pairs is not None
+    r3 = torch.empty_like(d.t3)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        res.compute(d, d.t3, r3)
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        res.compute(d, d.t3, r3)
+    for _ in range(2):
+        r3.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(r3, want)
+    assert res.status_ok()

@@ -255,7 +255,8 @@ class T3Residual:
             # the pair form reads W_vvvv's symmetry back to the host: not where the caller rules
             # host reads out
             self.pairs = contract.PairWvvvvT3(self.n3, nv, precision, device) if (
-                not woooo_pair_symmetric and contract.PairWvvvvT3.worthwhile(self.n3, nv)) else None
+                torch.device(device).type == "cuda" and not woooo_pair_symmetric
+                and contract.PairWvvvvT3.worthwhile(self.n3, nv)) else None
             self.ya = contract.Split(no * no * nv, no, k, device)
             self.yb = contract.Split(no * nv * nv, no, k, device)
             self.status = torch.zeros(1, dtype=torch.int32, device=device)

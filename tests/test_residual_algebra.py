@@ -77,3 +77,12 @@ def test_woooo_k_pieces():
     assert woooo_k_pieces(5, 6, limit=8 * 5 * 6 ** 3 + 1) == [8, 8, 8, 1]
     with pytest.raises(ValueError):
         woooo_k_pieces(4, 10, limit=100)
+
+
+def test_split_residual_constructs_without_a_device():
+    """The split precisions' residual and its operand plans can be built on the CPU at any nvir (the
+    pair form of W_vvvv.t3, from nvir = 60 on, keeps its pinned words for CUDA devices)."""
+    from dcc import t3_residual as tr
+    for nv in (7, 60):
+        res = tr.T3Residual(1, nv, "bf16x3", device="cpu")
+        assert res.pairs is None and res.xa.M == nv * nv

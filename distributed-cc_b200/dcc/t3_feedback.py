@@ -161,6 +161,9 @@ def intermediates_t3_add_(W_vooo, W_vvvo, t1_eris, X, nocc):
     return intermediates_t3_add_x_(W_vooo, W_vvvo, eris_slices(t1_eris, None, nocc)["oovv"], X)
 
 
+MAX_X = 128  # values of x to a launch: a grouped split holds DCC_GROUP_MAX = 256 operands, two per x
+
+
 class SplitFeedback:
     """The four T3 -> lower-order strings of the split-precision path as tcgen05 GEMMs on
     split operands (r1r2_add_t3_tri_ and intermediates_t3_add_t3_tri, distr_cc/rccsdt.py:
@@ -253,9 +256,10 @@ class SplitFeedback:
         return self.c.Split(rows, kind=self.kind, buffers=buf, pieces=ks, align=self.blk)
 
     def _group(self, group, xdtype):
-        """The grouped split and GEMM of the strings `group` (same columns and contraction) for
-        X of type xdtype: (grouped split, grouped GEMM, E element stride per x, rows M, columns N).
-        Their tables hold addresses of this object's buffers only; X and E are given per run."""
+        """The grouped splits and GEMMs of the strings `group` (same columns and contraction) for
+        X of type xdtype: ([(first x, end x, grouped split, grouped GEMM)], E element stride per x, rows M,
+        columns N), as many x to a launch as a table holds.  The tables hold addresses of this
+        object's buffers only; X and E are given per run."""
         key = (tuple(group), xdtype)
         if key not in self._groups:
             c, tm = self.c, self.terms[group[0]]
@@ -266,30 +270,38 @@ class SplitFeedback:
             A = self._operand(M, ks, Kp, self._ehi, self._elo)
             T = self._scratch[:M * N]
             es = A.hi.element_size()
-            split, gemm = [], []
             f32 = 1 if xdtype == torch.float32 else 0
-            for (op, fm, fk, sf) in ((B, tm["fn"], c.three(R1, R2, self.Sx, S1, S2), f32),
-                                     (A, c.lin(self.no * R1 * R2), c.lin(1), 0)):
-                for off, k, w in op.pieces:
-                    split.append([op.hi.data_ptr(), op.lo.data_ptr(), op.M, k, w, op.Kp, off] + list(c.as4(fm))
-                                 + list(c.as4(fk)) + [sf])
-            for off, _, w in A.pieces:
-                gemm.append([A.hi.data_ptr() + off * es, A.lo.data_ptr() + off * es, A.Kp, B.hi.data_ptr() + off * es,
-                             B.lo.data_ptr() + off * es, B.Kp, M, N, w, T.data_ptr(), 0] + list(c.as4(c.lin(N)))
-                            + list(c.as4(c.lin(1))))
-            self._groups[key] = (c.GroupedSplit(split, self.kind, self.dev),
-                                 c.GroupedGemm(gemm, np.ones(len(gemm)), self.kind, self.dev), R1 * R2, M, N)
+            xmap = c.three(R1, R2, self.Sx, S1, S2)
+            parts = []
+            for x0 in range(0, self.no, MAX_X):
+                x1 = min(x0 + MAX_X, self.no)
+                split, numel, gemm = [], [], []
+                for (op, fm, fk, sf) in ((B, tm["fn"], xmap, f32), (A, c.lin(self.no * R1 * R2), c.lin(1), 0)):
+                    for x in range(x0, x1):
+                        off, k, w = op.pieces[x]
+                        split.append([op.hi.data_ptr(), op.lo.data_ptr(), op.M, k, w, op.Kp, off] + list(c.as4(fm))
+                                     + list(c.as4(fk)) + [sf])
+                        numel.append(self.Sx if op is B else (M * self.no - x) * R1 * R2)
+                for off, _, w in A.pieces[x0:x1]:
+                    gemm.append([A.hi.data_ptr() + off * es, A.lo.data_ptr() + off * es, A.Kp, B.hi.data_ptr() + off * es,
+                                 B.lo.data_ptr() + off * es, B.Kp, M, N, w, T.data_ptr(), 0] + list(c.as4(c.lin(N)))
+                                + list(c.as4(c.lin(1))))
+                parts.append((x0, x1, c.GroupedSplit(split, self.kind, self.dev, numel),
+                              c.GroupedGemm(gemm, np.ones(len(gemm)), self.kind, self.dev)))
+            self._groups[key] = (parts, R1 * R2, M, N)
         return self._groups[key]
 
     def _contract(self, group, X, Ep, T):
-        """T = the products of the group's stacked E slices Ep with X, all x in two launches."""
-        split, gemm, estep, M, N = self._group(group, X.dtype)
+        """T = the products of the group's stacked E slices Ep with X, all x in two launches (two for
+        every MAX_X of them)."""
+        parts, estep, M, N = self._group(group, X.dtype)
         if Ep.dtype != f64 or not Ep.is_cuda or Ep.numel() != M * self.no * estep:
             raise ValueError("the E slices must be FP64 CUDA tensors of nocc / nvir extents")
         xs, es = self.Sx * X.element_size(), estep * Ep.element_size()
-        split.run([X.data_ptr() + x * xs for x in range(self.no)] + [Ep.data_ptr() + x * es for x in range(self.no)])
         T.zero_()
-        gemm.run(self.status)
+        for x0, x1, split, gemm in parts:
+            split.run([X.data_ptr() + x * xs for x in range(x0, x1)] + [Ep.data_ptr() + x * es for x in range(x0, x1)])
+            gemm.run(self.status)
 
     def _contract_pieces(self, group, X, Ep, T):
         c, tm = self.c, self.terms[group[0]]

@@ -83,6 +83,29 @@ def test_split_feedback_maps(no, nv):
         np.testing.assert_allclose(got.numpy(), want.numpy(), rtol=0, atol=1e-12 * want.abs().max().item())
 
 
+def _grouped_specs(monkeypatch, no, nv):
+    """[(split rows, GEMM rows)] of SplitFeedback's grouped launches, on the CPU."""
+    specs = []
+    monkeypatch.setattr(contract, "GroupedSplit", lambda rows, *a, **k: specs.append([rows]))
+    monkeypatch.setattr(contract, "GroupedGemm", lambda rows, *a, **k: specs[-1].append(rows))
+    sfb = fb.SplitFeedback(no, nv, "bf16x3", device="cpu")
+    for group in (("vovv", "wvooo"), ("ooov", "wvvvo"), ("wvooo",), ("wvvvo",)):
+        sfb._group(group, torch.float32)
+    return sfb, specs
+
+
+@pytest.mark.parametrize("no,nv", [(2, 3), (128, 1), (129, 1)])
+def test_grouped_feedback_tables(monkeypatch, no, nv):
+    """The grouped launches take any nocc: at most 256 operands and 256 products a table, every value
+    of x once."""
+    sfb, specs = _grouped_specs(monkeypatch, no, nv)
+    assert all(len(sp) <= 256 and len(gm) <= 256 and len(sp) == 2 * len(gm) for sp, gm in specs)
+    for at in range(4):
+        per = len(specs) // 4
+        rows = [r for _, gm in specs[per * at:per * (at + 1)] for r in gm]
+        assert len(rows) == no and len({r[0] for r in rows}) == no  # A pieces
+
+
 @pytest.mark.parametrize("no,nv", [(3, 5), (4, 7), (5, 4)])
 def test_r1_without_v_pass(oracle, no, nv):
     """r1's T3 part (distr_cc/rccsdt.py:262-296) from t3 directly: the permutations of V =

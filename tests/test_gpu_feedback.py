@@ -90,3 +90,29 @@ def test_r2_fock(mods, dtype, no, nv):
     want = r2 + 0.5 * torch.einsum("xa,xyzabc->yzbc", f, X.double())
     _c_rccsdt.t3_r2_fock_(r2, X, f, no, nv, 0.5)
     assert float((r2 - want).abs().max()) <= 1e-13 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("no,nv", [(1, 3), (4, 9), (6, 4), (3, 17), (129, 1)])
+def test_split_feedback(mods, no, nv, dtype):
+    """The grouped feedback of the split precisions against the FP64 strings (1e-5 of the largest entry:
+    a bf16 pair keeps an operand to 2^-18 = 4e-6, errors of random sign over the summed products): fewer and more virtual than occupied indices, and more
+    values of x than a table holds; also the W strings by themselves."""
+    fb, _ = mods
+    g = torch.Generator(device="cuda").manual_seed(no)
+    r = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda", generator=g)  # noqa: E731
+    X = r(no, no, no, nv, nv, nv).to(dtype)
+    E = {"vovv": r(nv, no, nv, nv), "ooov": r(no, no, no, nv), "oovv": r(no, no, nv, nv)}
+    z = lambda *s: torch.zeros(*s, dtype=torch.float64, device="cuda")  # noqa: E731
+    want = (z(no, no, nv, nv), z(nv, no, no, no), z(nv, nv, nv, no))
+    Xd = X.double()
+    fb.r2_add_t3_x_(want[0], z(no, nv), E["vovv"], E["ooov"], Xd)
+    fb.intermediates_t3_add_x_(want[1], want[2], E["oovv"], Xd)
+    s = fb.SplitFeedback(no, nv, "bf16x3")
+    got = tuple(torch.zeros_like(w) for w in want)
+    s.run(X, E, {"r2": got[0], "W_vooo": got[1], "W_vvvo": got[2]})
+    alone = tuple(torch.zeros_like(w) for w in want[1:])
+    s.run(X, {"oovv": E["oovv"]}, {"W_vooo": alone[0], "W_vvvo": alone[1]}, names=("wvooo", "wvvvo"))
+    assert int(s.status.item()) == 0
+    for a, b in list(zip(got, want)) + list(zip(alone, want[1:])):
+        assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())

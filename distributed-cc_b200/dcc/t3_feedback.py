@@ -186,7 +186,9 @@ class SplitFeedback:
     four digits to cancellation.  All pieces of both operands are split in one grouped launch and all
     x problems of a group run as one grouped GEMM (reductions in L2 into the scratch): a problem alone has
     36 tiles for 148 SMs at nocc=10 / nvir=90 (K = nvir^2), all ten 360.  The partial results
-    accumulate in an FP64 scratch T[row][column]
+    are added in no fixed order, but each is an FP32 number, so that their FP64 sum is exact, and its bits
+    the same from run to run, unless one is 2^-29 of another or less (twelve runs each at nocc=4 /
+    nvir=9, 6 / 40 and 10 / 64 gave equal bits).  They accumulate in an FP64 scratch T[row][column]
     (contiguous, so the epilogue writes whole rows; W_vvvo's own layout puts every element of an
     epilogue row in its own sector), and each string's rows are added to its output once, with a
     permutation.  One split buffer of X (nocc^2 nvir x nocc nvir^2 elements, two 2-byte pieces

@@ -251,12 +251,13 @@ class T3Residual:
             self.plan = s_plan(no, nv)
             self.xa = contract.Split(no * nv * nv, nv, k, device)
             self.xb = contract.Split(no * no * nv, nv, k, device)
-            self.wvvvv = contract.WvvvvT3(self.n3, nv, precision, device)
             # the pair form reads W_vvvv's symmetry back to the host: not where the caller rules
-            # host reads out
+            # host reads out.  Where it stands, the plain form and its operands are made when a W_vvvv
+            # first needs them
             self.pairs = contract.PairWvvvvT3(self.n3, nv, precision, device) if (
                 torch.device(device).type == "cuda" and not woooo_pair_symmetric
                 and contract.PairWvvvvT3.worthwhile(self.n3, nv)) else None
+            self._wvvvv = None if self.pairs is not None else contract.WvvvvT3(self.n3, nv, precision, device)
             self.ya = contract.Split(no * no * nv, no, k, device)
             self.yb = contract.Split(no * nv * nv, no, k, device)
             self.status = torch.zeros(1, dtype=torch.int32, device=device)
@@ -280,6 +281,13 @@ class T3Residual:
         self._small = self._A = self._sym = None
         if precision != "fp64" and torch.device(device).type == "cuda":
             self._small = self._small_split()
+
+    @property
+    def wvvvv(self):
+        """The plain form of W_vvvv.t3 (split precisions)."""
+        if self._wvvvv is None:
+            self._wvvvv = contract.WvvvvT3(self.n3, self.nv, self.precision, self.dev)
+        return self._wvvvv
 
     # ------------------------------------------------------------ pieces
     def _small_ops(self):
@@ -549,8 +557,7 @@ class T3Residual:
             return False
         if self.precision == "fp64":
             return True
-        return int(self.status.item()) == 0 and int(self.wvvvv.status.item()) == 0 and (
-            self.pairs is None or int(self.pairs.status.item()) == 0)
+        return all(int(x.status.item()) == 0 for x in (self, self._wvvvv, self.pairs) if x is not None)
 
 
 def update_t3_(t3, r3, d, nvir_active=None, norms=None, workspace=None, write_r3=True):

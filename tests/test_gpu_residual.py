@@ -345,3 +345,30 @@ def test_capture_without_oo_terms(mods):
         torch.cuda.synchronize()
         assert torch.equal(r3, want)
     assert res.status_ok()
+
+
+def test_one_form_of_wvvvv_in_memory(mods):
+    """A residual that takes the pair form of W_vvvv.t3 holds no more memory than one that takes the plain
+    form, and makes the plain form's operands only for a W_vvvv without the pair symmetry."""
+    syn, tr, _ = mods
+    no, nv = 3, 60
+    d = syn.make_inputs(no, nv, seed=9)
+    held = []
+    for plain in (True, False):
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        res = tr.T3Residual(no, nv, "bf16x3", woooo_pair_symmetric=plain)
+        r3 = res.compute(d, d.t3)
+        assert (res.pairs is None) == plain and res.status_ok()
+        del r3
+        held.append(torch.cuda.memory_allocated() - before)
+        if plain:
+            W = d.W_vvvv.clone()
+            W[0, 1, 0, 0] += 1.0
+            d.W_vvvv, keep = W, d.W_vvvv
+            want = res.compute(d, d.t3)
+            d.W_vvvv = keep
+            del res
+    assert held[1] <= held[0]
+    d.W_vvvv = W
+    assert torch.equal(res.compute(d, d.t3), want) and res.status_ok()

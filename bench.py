@@ -268,7 +268,8 @@ def t3_line(torch, ranks, contract, nocc, nvir, precision, steps, warmup, track_
         info["wvvvv_gemm_pipeline"] = {
             "kb_bytes": tuned[0], "stages": tuned[1], "group_m": tuned[2], "chosen_by": "dcc.autotune",
             "tile_n": tuned[3], "candidates_ms": {"%d/%d/%d/%d" % c: round(ms, 4) for c, ms in
-                                                  (autotune.timings(it.res.wvvvv.key()) or {}).items()}}
+                                                  (autotune.timings(it.res.wvvvv_key()) or {}).items()},
+            "form": "plain" if it.res.pairs is None else "pairs"}
         # the S GEMMs' tile width (128 x 256 or 128 x 128) and raster group, each tuned alone
         info["s_gemm_tiles"] = {
             name: {"chosen": "%d/%d/%d/%d" % cfg,

@@ -475,8 +475,10 @@ class WvvvvT3:
       'cd,abd'            = delta(b,d) F[c,e] t3[q,a,d,e]                          (third GEMM)
     so the first and third GEMMs take W plus those rank-deficient terms."""
 
-    def __init__(self, nblocks, nvir, kind="bf16x3", device="cuda"):
+    def __init__(self, nblocks, nvir, kind="bf16x3", device="cuda", key=None):
+        """key: the autotuner's key to apply (one of this form's own otherwise)."""
         self.n, self.nv, self.kind = int(nblocks), int(nvir), KIND[kind]
+        self._key = ("wvvvv_t3", self.n, self.nv, self.kind) if key is None else key
         K = nvir * nvir
         self.W = Split(K, K, self.kind, device)
         self.A = Split(self.n * nvir, K, self.kind, device)
@@ -485,7 +487,7 @@ class WvvvvT3:
         self.WF = None
 
     def key(self):
-        return ("wvvvv_t3", self.n, self.nv, self.kind)
+        return self._key
 
     def tune(self, scratch, W, t3, F=None):
         """Pick the GEMM tile and pipeline shape (tile columns, k-block width, ring depth, raster
@@ -570,6 +572,9 @@ class PairWvvvvT3:
         nocc=10 nvir=56 2.27 / 2.20, nocc=10 nvir=47 1.08 / 1.30, nocc=10 nvir=30 0.36 / 0.43)."""
         return nblocks > 0 and 60 <= nvir <= PairWvvvvT3.MAX_NVIR
 
+    def key(self):
+        return ("wvvvv_t3_pairs", self.n, self.nv, self.kind)
+
     def _pieces(self, pm):
         p, m = pm
         return (ctypes.c_void_p * 4)(p.hi.data_ptr(), p.lo.data_ptr(), m.hi.data_ptr(), m.lo.data_ptr())
@@ -581,7 +586,9 @@ class PairWvvvvT3:
     def __call__(self, r3, W, t3, alpha=1.0, F=None, scratch=None):
         """r3 += alpha (W_vvvv.t3 + F_vv.t3) and True; False, with r3 untouched, when W lacks the pair
         symmetry (one host read of two numbers).  scratch: a contiguous tensor whose bytes may hold
-        the FP32 results (six of rows x pairs; a buffer of this object otherwise)."""
+        the FP32 results (six of rows x pairs; a buffer of this object otherwise).  The GEMMs run under
+        the configuration tuned for key(), if one was."""
+        from . import autotune
         for x, name in ((r3, "r3"), (t3, "t3")):
             L.as_tensor(x, f64, name)
         nv, rows, npair = self.nv, self.rows, self.npair
@@ -611,15 +618,16 @@ class PairWvvvvT3:
                 self.own = torch.empty(need, dtype=torch.float32, device=self.dev)
             C = self.own
         C = C.view(3, 2, rows * npair)
-        for s in range(3):
-            if s:
-                self._split_t(t3, s)
-            for pm in range(2):
-                out = C[s, pm]
-                if s < 2:  # [q][pair][free]: the pass reads along the free index
-                    gemm_(self.w[pm], self.t[pm], out, lin(nv), two(nv, npair * nv, 1), 1.0, 0.0, self.status)
-                else:
-                    gemm_(self.t[pm], self.w[pm], out, lin(npair), lin(1), 1.0, 0.0, self.status)
+        with autotune.applied(self.key()):
+            for s in range(3):
+                if s:
+                    self._split_t(t3, s)
+                for pm in range(2):
+                    out = C[s, pm]
+                    if s < 2:  # [q][pair][free]: the pass reads along the free index
+                        gemm_(self.w[pm], self.t[pm], out, lin(nv), two(nv, npair * nv, 1), 1.0, 0.0, self.status)
+                    else:
+                        gemm_(self.t[pm], self.w[pm], out, lin(npair), lin(1), 1.0, 0.0, self.status)
         ptr = lambda pm: (ctypes.c_void_p * 3)(*[C[s, pm].data_ptr() for s in range(3)])  # noqa: E731
         L.check(_pair_add(ptr(0), ptr(1), L.ptr(r3), self.n, nv, float(alpha), L.stream_ptr()))
         return True

@@ -286,8 +286,12 @@ class T3Residual:
     def wvvvv(self):
         """The plain form of W_vvvv.t3 (split precisions)."""
         if self._wvvvv is None:
-            self._wvvvv = contract.WvvvvT3(self.n3, self.nv, self.precision, self.dev)
+            self._wvvvv = contract.WvvvvT3(self.n3, self.nv, self.precision, self.dev, key=self.wvvvv_key())
         return self._wvvvv
+
+    def wvvvv_key(self):
+        """The autotuner's key of this residual's W_vvvv.t3 GEMMs, in the form that its W_vvvv takes."""
+        return self.pairs.key() if self.pairs is not None else self._wvvvv.key()
 
     # ------------------------------------------------------------ pieces
     def _small_ops(self):
@@ -499,14 +503,19 @@ class T3Residual:
 
     def tune(self, d, t3):
         """Autotune the split precisions' GEMMs (the FP64 path has nothing to tune): the tile width,
-        pipeline shape and raster group of the W_vvvv.t3 GEMMs, then the tile width and raster
+        pipeline shape and raster group of the W_vvvv.t3 GEMMs in the form that d.W_vvvv takes (over
+        pairs, whose results are FP32, the pipeline follows the tile width), then the tile width and raster
         group of each S GEMM, each timed alone on this problem (their operands from one pass of
         s_ over d and t3; S is rebuilt by the next compute).  Returns the W_vvvv choice
         (k-block bytes, stages, group, tile columns); s_tuning() lists the others."""
         if self.precision == "fp64":
             return None
         from . import autotune
-        best = self.wvvvv.tune(torch.empty_like(t3), d.W_vvvv, t3, F=d.F_vv)
+        r3 = torch.empty_like(t3)
+        pairs = self.pairs is not None and self.pairs(r3, d.W_vvvv, t3, F=d.F_vv, scratch=self.S)
+        best = autotune.tune(self.wvvvv_key(), lambda: self.wvvvv_(r3, d, t3, scratch=self.S),
+                             cands=autotune.tile_candidates() if pairs else None)
+        del r3
         self.s_(d, t3)
         for name, (A, B, C, frow, fcol, alpha, beta, Kp) in self._sargs.items():
             old = autotune.get_config()

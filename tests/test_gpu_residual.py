@@ -372,3 +372,54 @@ def test_one_form_of_wvvvv_in_memory(mods):
     assert held[1] <= held[0]
     d.W_vvvv = W
     assert torch.equal(res.compute(d, d.t3), want) and res.status_ok()
+
+
+def test_tune_tunes_the_form_that_runs(mods, monkeypatch):
+    """T3Residual.tune times the GEMMs that compute() will launch for W_vvvv.t3 (over pairs here, the plain
+    ones for a W_vvvv without the pair symmetry), and each form runs under the choice, every
+    candidate within the split tolerance."""
+    syn, tr, _ = mods
+    from dcc import autotune, contract
+    old = autotune.get_config()
+    monkeypatch.setattr(autotune, "_cache", {})
+    monkeypatch.setattr(autotune, "_times", {})
+    try:
+        no, nv = 2, 66
+        d = syn.make_inputs(no, nv, seed=10)
+        want = tr.T3Residual(no, nv, "fp64").compute(d, d.t3)
+        res = tr.T3Residual(no, nv, "bf16x3")
+        seen, gemm = [], contract.gemm_
+        shapes = ({res.pairs.rows, res.pairs.npair}, {res.pairs.rows, nv * nv})
+
+        def spy(A, B, *a, **k):
+            for i, s in enumerate(shapes):
+                if {A.M, B.M} == s:
+                    seen.append((i, autotune.get_config()))
+            return gemm(A, B, *a, **k)
+
+        cfg = res.tune(d, d.t3)
+        assert autotune.chosen(res.wvvvv_key()) == cfg and set(autotune.timings(res.wvvvv_key())) == set(
+            autotune.tile_candidates())
+        assert res._wvvvv is None  # the plain form was neither built nor timed
+        autotune.set_config(*old)
+        monkeypatch.setattr(contract, "gemm_", spy)
+        for cand in autotune.tile_candidates():
+            autotune._cache[res.wvvvv_key()] = cand
+            del seen[:]
+            got = res.compute(d, d.t3)
+            assert seen == [(0, cand)] * 6 and autotune.get_config() == old
+            assert float((got - want).abs().max() / want.abs().max()) < TOL["bf16x3"]
+        monkeypatch.setattr(contract, "gemm_", gemm)
+        # a W_vvvv without the symmetry: the plain form is timed, over every pipeline
+        d.W_vvvv = d.W_vvvv + 0.01 * torch.rand_like(d.W_vvvv)
+        res = tr.T3Residual(no, nv, "bf16x3")
+        autotune._cache.pop(res.wvvvv_key())
+        cfg = res.tune(d, d.t3)
+        assert set(autotune.timings(res.wvvvv_key())) == set(autotune.candidates())
+        autotune.set_config(*old)
+        monkeypatch.setattr(contract, "gemm_", spy)
+        del seen[:]
+        res.compute(d, d.t3)
+        assert seen == [(1, cfg)] * 3
+    finally:
+        autotune.set_config(*old)

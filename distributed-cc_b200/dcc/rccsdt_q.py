@@ -361,13 +361,15 @@ class QEnergy:
 
     # ------------------------------------------------------------------ group data
     def _slabs(self, t3_abc, r, which=_SLABS, out=None):
-        """T3 slabs of the group / d-chunk r (FP64, filled on the device by one launch)."""
+        """T3 slabs of the group / d-chunk r (FP64, in one allocation, filled on the device by one launch)."""
         nv, no = self.nv, self.no
         rng = {"a": (r[0], r[1]), "b": (r[2], r[3]), "c": (r[4], r[5]), "d": (r[6], r[7])}
         out = {} if out is None else out
         ranges = [rng[s[1]] + rng[s[2]] for s in which]
         shapes = [(x1 - x0, y1 - y0, nv, no, no, no) for x0, x1, y0, y1 in ranges]
         sizes = [sh[0] * sh[1] * nv * no ** 3 for sh in shapes]
+        for s in which:
+            out.pop(s, None)  # the last chunk's, before this one's are allocated
         parts = torch.empty(sum(sizes), dtype=f64, device=self.dev).split(sizes)
         for s, sh, t in zip(which, shapes, parts):
             out[s] = t.view(sh)
@@ -553,11 +555,12 @@ class QEnergy:
         t2 = t2.contiguous()
         vvooT, t2T = self._transposed(er, t2)
         for (a0, a1, b0, b1, c0, c1), dlo, dhi in self._work(group_list, d_ranges):
-            slabs = {}
-            for d0, d1 in self._chunks(dlo, dhi):
+            slabs, chunks = {}, self._chunks(dlo, dhi)
+            if len(chunks) > 1:  # the slabs without d live as long as the group, those with d as a chunk
+                self._slabs(t3_abc, (a0, a1, b0, b1, c0, c1, c0, nv), which=("Sab", "Sac", "Sbc"), out=slabs)
+            for d0, d1 in chunks:
                 r = (a0, a1, b0, b1, c0, c1, d0, d1)
-                # the slabs without d once per group, with the first chunk's others
-                self._slabs(t3_abc, r, which=("Sad", "Sbd", "Scd") if slabs else _SLABS, out=slabs)
+                self._slabs(t3_abc, r, which=("Sad", "Sbd", "Scd") if len(chunks) > 1 else _SLABS, out=slabs)
                 if self.kind is None:
                     z, x = self._run_fp64(er, t2, slabs, r)
                 else:

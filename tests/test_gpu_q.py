@@ -114,3 +114,31 @@ def test_q_energy_split_jobs(mods, oracle, precision, n_jobs):
     tol = 1e-10 if precision == "fp64" else 1e-4
     assert abs(got[0] - want[0]) <= tol * abs(want[0])
     assert abs(got[1] - want[1]) <= tol * abs(want[1])
+
+
+def test_q_slabs_live_for_their_chunk(mods):
+    """The slabs over a d-chunk are freed with the chunk: a group run in three d-chunks holds the three
+    slabs of the group and three of one chunk at a time."""
+    gq, _ = mods
+    from dcc import _c_rccsdt, synthetic
+    no, nv, blk = 6, 24, 8
+    d = synthetic.make_inputs(no, nv, seed=3)
+    er = {"vvvo": d.W_vvvo, "vooo": d.W_vooo, "vvoo": d.eris_vvoo, "ovvo": d.W_ovvo, "ovov": d.W_ovov,
+          "vvvv": d.W_vvvv, "oooo": d.W_oooo}
+    t2 = d.t2.permute(2, 3, 0, 1).contiguous()
+    t3 = _c_rccsdt.redistribute_ijk_to_abc(d.t3, no, nv)
+    q = gq.QEnergy(no, nv, blk, "bf16x3", dchunk=blk)
+    g = gq.groups(nv, blk)[:1]  # a, b, c in [0, 8), d in three chunks of 8
+    assert len(q._chunks(g[0][4])) == 3
+    q.prepare(g)
+    want = q.run(er, t2, t3, d.e_occ, d.e_vir, g).clone()  # the transposed copies are made here
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    q.out.zero_()
+    got = q.run(er, t2, t3, d.e_occ, d.e_vir, g)
+    torch.cuda.synchronize()
+    slab = blk * blk * nv * no ** 3 * 8
+    small = 2 * 8 * (no * nv) ** 2 + (1 << 16)  # the transposed copies, rounding of allocations
+    assert torch.cuda.max_memory_allocated() - before <= 6 * slab + small
+    assert float((got - want).abs().max()) <= 1e-6 * float(want.abs().max()) and q.status_ok()

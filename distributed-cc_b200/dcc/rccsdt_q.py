@@ -354,7 +354,6 @@ class QEnergy:
         self.terms = group_terms()
         self._plans = {}
         self._arena = self._pool = None
-        self._vvooT = self._t2T = None
 
     def status_ok(self):
         return self.kind is None or int(self.status.item()) == 0
@@ -389,10 +388,8 @@ class QEnergy:
         return [(g,) + tuple(d_ranges[g]) for g in gl if g in d_ranges]
 
     def _transposed(self, er, t2):
-        if self._vvooT is None:
-            self._vvooT = er["vvoo"].permute(0, 2, 3, 1).contiguous()
-            self._t2T = t2.permute(0, 2, 3, 1).contiguous()
-        return self._vvooT, self._t2T
+        """vvoo and t2 in the order the group epilogue reads them."""
+        return er["vvoo"].permute(0, 2, 3, 1).contiguous(), t2.permute(0, 2, 3, 1).contiguous()
 
     # ------------------------------------------------------------------ FP64 path
     def _run_fp64(self, er, t2, slabs, r):

@@ -142,3 +142,22 @@ def test_q_slabs_live_for_their_chunk(mods):
     small = 2 * 8 * (no * nv) ** 2 + (1 << 16)  # the transposed copies, rounding of allocations
     assert torch.cuda.max_memory_allocated() - before <= 6 * slab + small
     assert float((got - want).abs().max()) <= 1e-6 * float(want.abs().max()) and q.status_ok()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "bf16x3"])
+def test_q_energy_object_takes_new_inputs(mods, precision):
+    """One QEnergy run on a second set of inputs adds that set's energies (a new object's, within the order
+    of its sums: 1e-10 in FP64, 1e-6 of the largest where products are FP32)."""
+    gq, _ = mods
+    from dcc import _c_rccsdt
+    no, nv, blk = 3, 7, 3
+    q, total, scale = gq.QEnergy(no, nv, blk, precision), np.zeros(2), 0.0
+    for seed in (31, 32):
+        er, t2, T, eo, ev = _inputs(no, nv, seed)
+        d = _device(er, t2, T, eo, ev, no)
+        t3 = _c_rccsdt.redistribute_ijk_to_abc(d[2], no, nv)
+        one = gq.QEnergy(no, nv, blk, precision).run(d[0], d[1], t3, d[3], d[4]).cpu().numpy()
+        got = q.run(d[0], d[1], t3, d[3], d[4]).cpu().numpy()
+        total, scale = total + one, max(scale, np.abs(one).max())
+        assert np.abs(got - total).max() <= (1e-10 if precision == "fp64" else 1e-6) * scale
+    assert q.status_ok()

@@ -116,3 +116,20 @@ def test_split_feedback(mods, no, nv, dtype):
     assert int(s.status.item()) == 0
     for a, b in list(zip(got, want)) + list(zip(alone, want[1:])):
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("no,nv", [(3, 5), (255, 1), (256, 1), (260, 2)])
+def test_fock_term(no, nv):
+    """The iteration's f_ov term on either side of the one-launch kernel's limit (nocc < 256) against the
+    einsum in FP64 (beyond it the products are those of X's type: 1e-6 of the largest entry)."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from types import SimpleNamespace
+    from dcc.t3_iteration import T3Iteration
+    g = torch.Generator(device="cuda").manual_seed(no)
+    X = torch.randn((no,) * 3 + (nv,) * 3, dtype=torch.float32, device="cuda", generator=g)
+    f = torch.randn(no, nv, dtype=torch.float64, device="cuda", generator=g)
+    r2 = torch.randn(no, no, nv, nv, dtype=torch.float64, device="cuda", generator=g)
+    want = r2 + 0.5 * (f.view(no, 1, nv, 1) * X.view(no, no * no, nv, nv * nv)).sum((0, 2)).view_as(r2)
+    T3Iteration._fock_term_(SimpleNamespace(no=no, nv=nv, _X=X), r2, f)
+    assert float((r2 - want).abs().max()) <= 1e-6 * float(want.abs().max())

@@ -282,3 +282,24 @@ def test_unpack_all_large_blocks(nv):
     assert torch.equal(T[0], want)
     want = 2.0 * want - want.transpose(0, 1) - want.transpose(0, 2) - want.transpose(0, 3)
     assert torch.equal(Ts[0], want)
+
+
+@pytest.mark.parametrize("own", ["spin4", "forms", "both"])
+@pytest.mark.parametrize("no,nv", [(4, 5), (7, 11)])
+def test_compute_r4_tri_callers_forms(oracle, no, nv, own):
+    """compute_r4_tri_ with the caller's P4_201 (the unpack and the spin summation apart) and with the
+    caller's block forms (the W_ovov / W_voov strings in pair mode over the sparse pair lists, which no
+    other route takes) against the oracle, as test_compute_r4_tri."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from dcc import t4_residual, _c_rccsdt_q, _c_rccsdtq
+    d, want = _case(oracle, no, nv)
+    t = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in d.items()}
+    spin4 = lambda A: _c_rccsdt_q.t4_spin_summation_inplace_(A, A.numel() // nv ** 4, nv, "P4_201", 1.0, 0.0)  # noqa: E731
+    forms = lambda x: _c_rccsdtq.t4_forms_batched(x, nv)  # noqa: E731
+    r4 = torch.zeros_like(t["t4"])
+    t4_residual.compute_r4_tri_(r4, t["eris"], t["F_vv"], t["W_vvvo"], t["W_vooo"], t["W_vvvv"], t["W_oooo"],
+                                t["W_ovov"], t["t2"], t["t3"], t["t4"], no, "fp64", F_oo=t["F_oo"], W_ovvo=t["W_ovvo"],
+                                spin4=spin4 if own != "forms" else None, forms=forms if own != "spin4" else None)
+    assert np.abs(r4.cpu().numpy() - want).max() <= 1e-11 * np.abs(want).max()
+    assert int(t4_residual.fused_status(r4.device).item()) == 0

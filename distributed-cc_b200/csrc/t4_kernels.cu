@@ -131,8 +131,8 @@ __global__ void k_unpack_t4(const double *src, double *out, int64_t loc, int ax0
 // axis of the stored block that axis m of the ordering is.  With SMEM the block is staged at an
 // odd pitch (the four strided reads of a warp then hit distinct banks) and read from L1/L2
 // otherwise.  Bound by the writes (16 bytes per element of the ordered space, 0.09 ms at 6.5 TB/s at
-// nocc=7, nvir=11) and the latency of one staged block per SM: 0.235 ms there, against 2.0 ms for a
-// gather and a scatter per axis permutation, a copy and the orbit kernel (50 launches).
+// nocc=7, nvir=11) and the latency of its strided reads: 0.196 ms there, against 2.0 ms for a gather
+// and a scatter per axis permutation, a copy and the orbit kernel (50 launches).
 //
 // The digits of an element come from a multiplied reciprocal (Granlund and Montgomery, 1994): with
 // 2^(l-1) < nv <= 2^l and m = ceil(2^(31+l) / nv), which fits 32 bits, x / nv = (x m) >> (31 + l) for
@@ -289,10 +289,16 @@ extern "C" int dcc_t4_unpack_all(const double *t4, const int32_t *src, const int
     const T4Magic mg = t4_magic((int)nvir);
     const int pitch = (int)(nvir | 1);
     const size_t smem = (size_t)pitch * pitch * pitch * pitch * sizeof(double);
-    const int threads = nvir >= 9 ? 512 : 256;
-    // staged while two of the blocks, or one and its padding, fit an SM: nvir <= 11
-    if (smem <= 120 * 1024) {
-        cudaFuncSetAttribute(k_t4_unpack_all<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024);
+    // Staged while several blocks fit an SM (52 KB at nvir = 8 and 9, four of them), read through L1
+    // above: staged / direct in ms, 512 threads, nocc=9 nvir=8 0.107 / 0.198, nvir=9 0.161 / 0.178,
+    // nvir=10 (one block of 117 KB an SM) 0.485 / 0.317; nocc=7 nvir=11 0.242 / 0.196; nvir=13 (nocc=6)
+    // 0.281 / 0.271.  512 threads from nvir = 8 on (256 there: 0.123 at nocc=9 nvir=8, 0.197 at
+    // nvir=9); smaller blocks have too few elements for them (nocc=10: nvir=3 0.027 against 0.016 with 256,
+    // nvir=7 0.095 against 0.090).
+    const int threads = nvir >= 8 ? 512 : 256;
+    constexpr size_t staged_max = 72 * 1024;
+    if (smem <= staged_max) {
+        cudaFuncSetAttribute(k_t4_unpack_all<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged_max);
         k_t4_unpack_all<true><<<(unsigned)norder, threads, smem, as_stream(stream)>>>(t4, src, rank, T, Ts, mg, pitch);
     } else {
         k_t4_unpack_all<false><<<(unsigned)norder, threads, 0, as_stream(stream)>>>(t4, src, rank, T, Ts, mg, pitch);

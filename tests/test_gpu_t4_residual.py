@@ -166,9 +166,9 @@ def test_fused_strings_checks():
         assert torch.isfinite(r4).all(), bad
 
 
-@pytest.mark.parametrize("no,nv", [(3, 1), (2, 5), (4, 10), (3, 11), (3, 12), (3, 13)])
+@pytest.mark.parametrize("no,nv", [(3, 1), (2, 5), (3, 8), (3, 9), (4, 10), (3, 11), (3, 12), (3, 13)])
 def test_unpack_all_orderings(no, nv):
-    """t4_unpack_all on either side of the staged blocks' size limit (nvir 11), even and odd
+    """t4_unpack_all on either side of the staged blocks' size limit (nvir 9), even and odd
     extents: T equal to the indexed unpack, Ts to the P4_201 kernel on it (== : the same products
     and sums; a signed zero may differ)."""
     if not torch.cuda.is_available():

@@ -1226,9 +1226,12 @@ static int gemm_split3(const void *A_hi, const void *A_lo, int64_t lda, const vo
     // (two per TMEM lane quarter) double its memory parallelism; the ring then
     // is three 64-byte stages to make room for their staging buffers.
     const int esz = kind == 0 ? 2 : 4;
-    // an FP32 C takes the wide epilogue, unless it is written plainly (beta = 0) after a long
-    // contraction, whose MMAs hide a narrow one: then a fourth stage instead
-    const bool f32_long = c_f32 && beta == 0.0 && Kp >= 2048 && !narrow;
+    // An FP32 C takes the wide epilogue, unless it is written plainly (beta = 0) after a long
+    // contraction, whose MMAs hide a narrow one: then a fourth stage instead.  The six pair GEMMs of
+    // W_vvvv.t3, ms wide / fourth stage by 64-byte k-blocks: bf16 66 (nocc=10 nvir=64) 1.77 / 2.00, 128 (nocc=10
+    // nvir=90) 8.24 / 8.51, 138 (nocc=8 nvir=93) 5.67 / 5.75, 158 (nocc=5 nvir=100) 2.36 / 2.30, 198 (nocc=4
+    // nvir=112) 2.80 / 2.69; tf32 130 (nocc=10 nvir=64) 3.25 / 3.20, 256 (nocc=6 nvir=90) 4.45 / 4.11.
+    const bool f32_long = c_f32 && beta == 0.0 && Kp * esz >= 150 * 64 && !narrow;
     const bool wide_epi = Kp <= 4096 || c_f32;
     const int kb = (wide_epi || narrow) ? 64 : cfg.kb_bytes;
     const int tn = narrow ? 128 : GN;

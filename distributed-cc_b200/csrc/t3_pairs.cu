@@ -7,9 +7,9 @@
 // Each of the three strings becomes two split GEMMs of nvir(nvir+1)/2 columns and as long a
 // contraction in place of one of nvir^2 and nvir^2.  Here: the operands t+-, W+- as K-major two-piece
 // splits (sums and differences in FP64, then split), and the pass that adds the six FP32 results
-// (the accumulation type of the products) into r3 in FP64.  nocc=10, nvir=90: the six GEMMs 8.4 ms in
-// place of 17.4 (1.41 PFLOP/s of bf16 products either way), the three strings together 13.9 in
-// place of 21.5; the relative error of the result about half (2.2e-5 against 4.4e-5 at nvir=112 on
+// (the accumulation type of the products) into r3 in FP64.  nocc=10, nvir=90: the six GEMMs 8.2 ms in
+// place of 17.4 (1.4 PFLOP/s of bf16 products either way), the three strings together 12.5 in
+// place of 19.5; the relative error of the result about half (2.2e-5 against 4.4e-5 at nvir=112 on
 // random data: the FP32 accumulation is half as long).
 #include "dcc_common.cuh"
 #include "split_util.cuh"

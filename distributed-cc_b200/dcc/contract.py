@@ -567,9 +567,10 @@ class PairWvvvvT3:
     @staticmethod
     def worthwhile(nblocks, nvir):
         """Whether the pair form is the faster one: from nvir = 60 on, where the products outweigh the
-        pass over the results (ms of all three strings, plain / pairs: nocc=10 nvir=90 21.5 / 13.9,
-        nocc=6 nvir=93 6.7 / 4.5, nocc=10 nvir=60 3.16 / 2.78, nocc=5 nvir=64 0.90 / 0.89; below,
-        nocc=10 nvir=56 2.27 / 2.20, nocc=10 nvir=47 1.08 / 1.30, nocc=10 nvir=30 0.36 / 0.43)."""
+        pass over the results (ms of all three strings, plain / pairs: nocc=10 nvir=90 19.5 / 12.5,
+        nocc=6 nvir=93 6.74 / 4.06, nocc=4 nvir=112 6.65 / 4.42, nocc=10 nvir=60 3.26 / 2.76, nocc=5 nvir=64
+        0.94 / 0.90; below, nocc=10 nvir=56 2.30 / 2.21, nocc=10 nvir=47 1.15 / 1.32, nocc=10 nvir=30
+        0.46 / 0.52)."""
         return nblocks > 0 and 60 <= nvir <= PairWvvvvT3.MAX_NVIR
 
     def key(self):

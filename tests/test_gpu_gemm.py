@@ -246,7 +246,7 @@ def test_split_of_fp32_source(C, kind, maps):
 
 
 @pytest.mark.parametrize("kind", ["bf16x3", "tf32x3"])
-@pytest.mark.parametrize("nblk,nv", [(1, 1), (3, 2), (2, 7), (3, 16), (2, 31), (2, 33), (1, 64), (1, 112)])
+@pytest.mark.parametrize("nblk,nv", [(1, 1), (3, 2), (2, 7), (3, 16), (2, 31), (2, 33), (1, 64), (1, 96), (1, 97), (1, 112)])
 def test_pair_wvvvv(C, kind, nblk, nv):
     """W_vvvv.t3 + F_vv.t3 over symmetric / antisymmetric pairs against the FP64 einsums: remainders of
     every tile (pairs, rows, k-blocks, 32-wide column chunks) and the largest nvir; error within

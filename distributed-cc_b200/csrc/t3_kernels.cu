@@ -1021,8 +1021,6 @@ __device__ __forceinline__ int abc_case(int a, int b, int c, int s[3]) {
     return cs;
 }
 
-// One CTA per (ia, ib, c) block of nocc^3: load the ABC block, write it with
-// the occupied axes permuted.
 // The T3 slabs of one (Q) task group, T[X, Y, :, i, j, k] for up to six (X, Y) ranges, in one
 // launch.  A slab block (x, y, c) is one stored occupied cube with its axes permuted.
 constexpr int FILL_SLABS = 6;
@@ -1578,6 +1576,7 @@ extern "C" int dcc_redistribute_ijk_to_abc(const double *t3_ijk, double *t3_abc,
 static int fill_launch(FillTable &t, const int64_t *ba, int64_t nvir, int64_t nocc, const double *t3_abc,
                        void *stream) {
     const int64_t o3 = nocc * nocc * nocc;
+    // the range of these entries (nocc <= 29) is older than this kernel, which does not need it
     DCC_REQUIRE(o3 * 8 <= 200 * 1024, DCC_ERR_UNSUPPORTED, "nocc^3 blocks above 200 KiB");
     int64_t nwork = 0;
     for (int p = 0; p < t.n; p++) {

@@ -226,8 +226,9 @@ def _group_digits(order, size, strides):
 def _digit_orders(idx, size, strides, max_digits=4, prefer=None):
     """An order of idx whose digit grouping has at most max_digits digits (None if none).
     prefer: a stride table; an order whose fastest index is the contiguous one of that tensor is
-    taken first (an output tile is then written in runs: 'ijkabc,laid->jkldcb' of the adjoint at
-    nocc=6 / nvir=40 0.35 -> 0.08 ms)."""
+    taken first (an output tile is then written in runs).  Of the adjoint's 25 contractions it changes
+    'ijkabc,lbid->jkldca' and 'ijkabc,laid->jkldcb' (ms with their splits 0.46 -> 0.20 at nocc=6 /
+    nvir=40, 0.20 -> 0.10 at 5 / 31, 0.096 -> 0.080 at 4 / 12); the others stay within 4 % either way."""
     import itertools
     cand = [list(idx)] + [list(p) for p in itertools.permutations(idx)] if len(idx) <= 6 else [list(idx)]
     if prefer is not None and any(prefer[c] == 1 for c in idx):

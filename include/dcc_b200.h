@@ -231,7 +231,7 @@ DCC_API int dcc_redistribute_ijk_to_abc(const double *t3_ijk, double *t3_abc, in
 
 /* The slabs target[p] = T[a0..a1, b0..b1, :, i, j, k] ([a1-a0][b1-b0][nvir][nocc]^3 each, DEVICE) of
  * up to six ranges (a0, a1, b0, b1) = ranges[4p..4p+3] (targets and ranges HOST arrays), as
- * dcc_fill_t3_from_abc fills one, in one launch. */
+ * dcc_fill_t3_from_abc fills one, in one launch (nocc <= 29, as there). */
 DCC_API int dcc_fill_t3_slabs(double *const *targets, const int64_t *ranges, int nslab, int64_t nvir, int64_t nocc,
                               const double *t3_abc, void *stream);
 
@@ -239,7 +239,7 @@ DCC_API int dcc_fill_t3_slabs(double *const *targets, const int64_t *ranges, int
  * b in [b0,b1), all c, from ABC storage t3_abc[g][x][y][z] with the occupied
  * axes permuted by the virtual ordering case.  Replaces fill_t3_from_ptr_array
  * (src/rccsdt_q.c:655-828); at one rank every ABC block is local, so the
- * pointer table becomes one contiguous array. */
+ * pointer table becomes one contiguous array.  nocc <= 29. */
 DCC_API int dcc_fill_t3_from_abc(double *target, int64_t a0, int64_t a1, int64_t b0, int64_t b1, int64_t nvir,
                          int64_t nocc, const double *t3_abc, int64_t ld_b, void *stream);
 

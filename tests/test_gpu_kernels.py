@@ -322,7 +322,7 @@ def test_fill_t3_from_abc(C, oracle, nocc, nvir, blk):
 
 @pytest.mark.parametrize("nocc,nvir", [(1, 3), (2, 5), (5, 9), (8, 6), (9, 6), (17, 3)])
 def test_fill_t3_slabs(C, nocc, nvir):
-    """Six slabs in one launch (an empty one among them, cubes of either kernel's size) equal the
+    """Six slabs in one launch (an empty one among them, cubes of less and more than a warp's elements) equal the
     one-slab fills, which test_fill_t3_from_abc holds against the oracle."""
     cq = C[1]
     rng = np.random.default_rng(nocc)

@@ -380,11 +380,15 @@ def check_grouped_spans(spec, numel):
     _check_span asks of a single split's tensor)."""
     if len(numel) != len(spec):
         raise ValueError("need the elements of %d sources" % len(spec))
-    for p, (row, n) in enumerate(zip(spec, numel)):
-        M, K, fm, fk = int(row[2]), int(row[3]), [int(x) for x in row[7:14]], [int(x) for x in row[14:21]]
-        if any(x < 0 for x in fm[3:] + fk[3:]):
+
+    def top(R1, R2, R3, S0, S1, S2, S3, m):  # _max_offset of the indices up to m
+        return m // (R1 * R2 * R3) * S0 + min(R1 - 1, m // (R2 * R3)) * S1 + min(R2 - 1, m // R3) * S2 + \
+            min(R3 - 1, m) * S3
+
+    for p, (row, n) in enumerate(zip(np.asarray(spec, dtype=np.int64).tolist(), numel)):
+        if min(row[10:14] + row[17:21]) < 0:
             raise ValueError("operand %d: negative map strides" % p)
-        if M > 0 and K > 0 and _max_offset(fm, M) + _max_offset(fk, K) >= n:
+        if row[2] > 0 and row[3] > 0 and top(*row[7:14], row[2] - 1) + top(*row[14:21], row[3] - 1) >= n:
             raise ValueError("operand %d: the address maps reach past its source" % p)
 
 

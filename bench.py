@@ -689,7 +689,8 @@ def main():
     hbm, bf16, bf16_sus, src = peaks()
     peak_useful = bf16_sus / 3.0  # three bf16 products per FP64-equivalent flop
     achieved = flops_launch / (gemm_avg * 1e-3) / 1e12 if gemm_avg else None
-    traffic = profile_traffic("gemm_split3_wvvvv_nocc%d_nvir%d" % (no, nv))
+    form = "pairs" if (mix.get("wvvvv_gemm_pipeline") or {}).get("form") == "pairs" else "wvvvv"
+    traffic = profile_traffic("gemm_split3_%s_nocc%d_nvir%d" % (form, no, nv))
 
     value = ranks.job_seconds_per_iteration(mix["ms_total"], args.steps, world)  # whole job, replicas
     line = {

@@ -31,10 +31,10 @@ __global__ void k_r1_mix(const double *__restrict__ E, double *__restrict__ K, i
 
 // CTA (q, x0): the sums of block q over x in [x0, x0 + 4), one warp per y, lanes along z (NZ tiles
 // of 32).  A warp keeps B of its lanes' z in registers and A of its y for the four x; C comes
-// broadcast from shared memory.  part[item][m][v] gets the CTA's share of R_m[v].  Bound by the
-// one read of t3 (and the reads of A, a quarter of it, from L2), whose loads run one y ahead of
-// their use: nocc=10, nvir=90 (1.28 GB) 0.45 ms, 2.8 TB/s (0.61 without the loads ahead); the three
-// batched GEMMs with three right-hand sides and the seventy launches around them took 1.9 ms.
+// broadcast from shared memory.  part[item][m][v] gets the CTA's share of R_m[v].  Bound by
+// issue and load latency at eight warps an SM (229 registers; DRAM 32 %, FP64 pipe 23 % busy at nocc=6,
+// nvir=90), so the loads run one y ahead of their use: nocc=10, nvir=90 (1.28 GB, A a quarter more from
+// L2) 0.45 ms, 2.8 TB/s (0.61 without the loads ahead); the three batched GEMMs with three right-hand sides and the seventy launches around them took 1.9 ms.
 template <int NZ>
 __global__ void __launch_bounds__(R1_THREADS, 1)
     k_r1_t3(const double *__restrict__ t3, const double *__restrict__ K, const int32_t *__restrict__ ijk, int nocc,

@@ -96,8 +96,9 @@ __device__ __forceinline__ void plane_each(const double *__restrict__ src, int64
 
 // t+- of rows (q, f) whose plane (d, e) has e contiguous: t3[q][f fs + d ds + e].  One CTA per row:
 // the plane is staged at an odd pitch (both orders read free of bank conflicts), then written as
-// 16-byte packs.  Bound by DRAM (8 bytes read, 4 written per element of t3: 0.3 ms at 6.5 TB/s at
-// nocc=10, nvir=90) and the conversions: 0.64 ms there.
+// 16-byte packs.  Bound by the latency of a plane's loads at three CTAs an SM (its shared memory; DRAM
+// 35 % busy at nocc=6, nvir=90): nocc=10, nvir=90 0.64 ms, 0.3 at 6.5 TB/s (8 bytes read, 4 written per
+// element of t3).
 template <int KIND>
 __global__ void __launch_bounds__(PR_THREADS) k_pair_rows(const double *__restrict__ t3, const uint16_t *__restrict__ tab,
                                                           int nv, int64_t fs, int64_t ds, PairOut o) {
@@ -224,8 +225,9 @@ __global__ void __launch_bounds__(PR_THREADS) k_pair_w(const double *__restrict_
 // of the unordered pair: C1 as [q][pair][c], C2 as [q][pair][b], C3 as [q][a][pair], so that all but
 // the transposition of C2 (through shared memory) is read along rows, and a block's 90 or so CTAs
 // share its 9 MB of results in L2 (with q innermost, [pair][q][c], every 360-byte run was its own
-// DRAM page: 4.0 ms).  One CTA per plane (q, a), two rows' loads in flight a lane.  Bound by DRAM:
-// nocc=10, nvir=90 (4.5 GB) 2.16 ms.
+// DRAM page: 4.0 ms).  One CTA per plane (q, a), two rows' loads in flight a lane.  Bound by
+// the latency of its loads at two CTAs an SM (registers and the transposed plane; DRAM 26 % busy at
+// nocc=6, nvir=90): nocc=10, nvir=90 (4.5 GB) 2.16 ms.
 struct PairC {
     const float *p[3], *m[3];
 };

@@ -130,8 +130,8 @@ __global__ void k_unpack_t4(const double *src, double *out, int64_t loc, int ax0
 // src[o] = its stored block (-1: not stored, zeros) and rank[o] packs, one nibble per axis m, the
 // axis of the stored block that axis m of the ordering is.  With SMEM the block is staged at an
 // odd pitch (the four strided reads of a warp then hit distinct banks) and read from L1/L2
-// otherwise.  Bound by the writes (16 bytes per element of the ordered space, 0.09 ms at 6.5 TB/s at
-// nocc=7, nvir=11) and the latency of its strided reads: 0.196 ms there, against 2.0 ms for a gather
+// otherwise.  Bound by the requests of its strided reads (L2 60 % busy, DRAM 34 % at nocc=7, nvir=11,
+// where the writes, 16 bytes per element of the ordered space, take 0.09 ms at 6.5 TB/s): 0.196 ms there, against 2.0 ms for a gather
 // and a scatter per axis permutation, a copy and the orbit kernel (50 launches).
 //
 // The digits of an element come from a multiplied reciprocal (Granlund and Montgomery, 1994): with

@@ -21,8 +21,8 @@
 // A run whose GEMM has one row (the F_oo / W_oooo strings: no output letter in W) is a sum
 // of scaled vectors and runs on the FP64 lanes.
 //
-// What bounds it: operand loads (L1) and the FP64 matrix pipe; the contractions are short
-// (7 to 121 summed values).  Measured (nocc=7, nvir=11, 161 blocks, B200): the kernel 3.5 ms, against
+// What bounds it: the latency of operand loads at sixteen warps an SM (16 GB from L2 at nocc=7,
+// nvir=11, 17 % of its rate; DRAM 4 %); the contractions are short (7 to 121 summed values).  Measured (nocc=7, nvir=11, 161 blocks, B200): the kernel 3.5 ms, against
 // 8.3 ms with FP64 lanes, one barrier and one shared-memory update per string and pair; at
 // nocc=5, nvir=8 0.47 against 2.2 ms.
 //

@@ -12,6 +12,8 @@
     python profile_cases.py t3half [--reps 3] [--nocc 15 --nvir 93] [--kind bf16x3|fp64] [--breakdown]
     python profile_cases.py t4     [--reps 3] [--kind bf16x3|fp64] [--breakdown]
     python profile_cases.py oddnv  [--reps 3] [--nocc 5 --nvir 93] [--time] [--passes 0,1,...]
+    python profile_cases.py pairs  [--reps 3] [--nocc 6 --nvir 90] [--kind bf16x3]
+    python profile_cases.py feedback [--reps 3] [--nocc 6 --nvir 90]
 
 Each case builds its inputs once and launches the kernel `reps` times, so a
 profiler can skip the warm-up launches and capture the last one.  Sizes are
@@ -44,6 +46,39 @@ def case_gemm(kind, reps, nocc=10, nvir=90):
         contract.gemm_(op.A, op.W, r3, er, ec, 1.0, 1.0, op.status)
     torch.cuda.synchronize()
     assert int(op.status.item()) == 0
+
+
+def case_pairs(kind, reps, nocc=6, nvir=90):
+    """W_vvvv.t3 over symmetric / antisymmetric pairs: per repetition the two operand passes of W and t3,
+    six GEMMs and the pass that adds their results to r3."""
+    from dcc import contract
+    n3, nv = nocc * (nocc + 1) * (nocc + 2) // 6, nvir
+    g = torch.Generator(device="cuda").manual_seed(0)
+    t3 = torch.randn(n3, nv, nv, nv, dtype=torch.float64, device="cuda", generator=g) * 1e-3
+    W = torch.randn(nv, nv, nv, nv, dtype=torch.float64, device="cuda", generator=g) * 0.1
+    W = (W + W.permute(1, 0, 3, 2)).contiguous()
+    r3 = torch.zeros_like(t3)
+    op = contract.PairWvvvvT3(n3, nv, kind)
+    for _ in range(reps):
+        assert op(r3, W, t3)
+    torch.cuda.synchronize()
+    assert int(op.status.item()) == 0
+
+
+def case_feedback(reps, nocc=6, nvir=90):
+    """r1's T3 part over canonical blocks and r2's Fock term over an FP32 X."""
+    from dcc import _c_rccsdt
+    from dcc.synthetic import canonical_ijk
+    ijk = torch.tensor(canonical_ijk(nocc), dtype=torch.int32, device="cuda")
+    t3 = torch.randn(ijk.shape[0], nvir, nvir, nvir, dtype=torch.float64, device="cuda")
+    X = torch.randn(nocc ** 3, nvir, nvir, nvir, dtype=torch.float32, device="cuda")
+    E = torch.randn(nocc, nocc, nvir, nvir, dtype=torch.float64, device="cuda")
+    f = torch.randn(nocc, nvir, dtype=torch.float64, device="cuda")
+    r1, r2 = torch.zeros_like(f), torch.zeros_like(E)
+    for _ in range(reps):
+        _c_rccsdt.t3_r1_(r1, t3, E, ijk, nocc)
+        _c_rccsdt.t3_r2_fock_(r2, X, f, nocc, nvir, 0.5)
+    torch.cuda.synchronize()
 
 
 def case_p3(reps, nvir=90, op="p3", time=False):
@@ -420,7 +455,7 @@ def case_t4(reps, kind="bf16x3", breakdown=False):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("case", choices=["gemm", "p3", "update", "q", "gather", "xgemm", "oogemm", "unpack", "qgroup",
-                                         "t4", "t3iter", "qsample", "t3half", "oddnv", "splits"])
+                                         "t4", "t3iter", "qsample", "t3half", "oddnv", "splits", "pairs", "feedback"])
     ap.add_argument("--kind", default="bf16x3")
     ap.add_argument("--reps", type=int, default=3)
     ap.add_argument("--nocc", type=int, default=None, help="occupied orbitals (xgemm, oogemm, gather, unpack)")
@@ -438,6 +473,10 @@ def main():
         case_gemm(a.kind, a.reps, a.nocc or 10, a.nvir or 90)
     elif a.case == "p3":
         case_p3(a.reps, a.nvir or 90, a.op, a.time)
+    elif a.case == "pairs":
+        case_pairs(a.kind, a.reps, a.nocc or 6, a.nvir or 90)
+    elif a.case == "feedback":
+        case_feedback(a.reps, a.nocc or 6, a.nvir or 90)
     elif a.case == "update":
         case_update(a.reps)
     elif a.case == "t4":

@@ -131,8 +131,9 @@ __global__ void k_unpack_t4(const double *src, double *out, int64_t loc, int ax0
 // axis of the stored block that axis m of the ordering is.  With SMEM the block is staged at an
 // odd pitch (the four strided reads of a warp then hit distinct banks) and read from L1/L2
 // otherwise.  Bound by the requests of its strided reads (L2 60 % busy, DRAM 34 % at nocc=7, nvir=11,
-// where the writes, 16 bytes per element of the ordered space, take 0.09 ms at 6.5 TB/s): 0.196 ms there, against 2.0 ms for a gather
-// and a scatter per axis permutation, a copy and the orbit kernel (50 launches).
+// where the writes, 16 bytes per element of the ordered space, take 0.09 ms at 6.5 TB/s): 0.196 ms
+// there, against 2.0 ms for a gather and a scatter per axis permutation, a copy and the orbit kernel
+// (50 launches).
 //
 // The digits of an element come from a multiplied reciprocal (Granlund and Montgomery, 1994): with
 // 2^(l-1) < nv <= 2^l and m = ceil(2^(31+l) / nv), which fits 32 bits, x / nv = (x m) >> (31 + l) for

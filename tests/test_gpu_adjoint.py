@@ -83,3 +83,22 @@ def test_split_backward(adj):
         grads[prec] = [x.grad for x in xa]
     for a, b in zip(grads["bf16x3"], grads["fp64"]):
         assert float((a - b).abs().max()) <= 1e-4 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("no,nv", [(3, 8), (4, 12)])
+def test_split_t3_gradient_keeps_f_apart(adj, no, nv):
+    """Where F_oo / F_vv dominate, t3's gradient in tf32x3 is exact to the 22 bits that two tf32 pieces
+    carry: F's short sums are not rounded along with W's longer ones (joined to them the error is
+    1.5 and 2.9 times the bound, apart 0.5 and 0.7)."""
+    xs, d = _inputs(no, nv, seed=5)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    lam = torch.randn(d.t3.shape, dtype=torch.float64, device="cuda", generator=g)
+    for i in (2, 3):  # F of order one, W a thousandth of it
+        xs[i] = torch.randn(xs[i].shape, dtype=torch.float64, device="cuda", generator=g)
+    for i in range(4, 10):
+        xs[i] = xs[i] * (1e-3 / xs[i].abs().max())
+    got = {}
+    for prec in ("fp64", "tf32x3"):
+        xa = [x.clone().requires_grad_(True) for x in xs]
+        got[prec] = torch.autograd.grad((lam * adj.t3_residual_fn(*xa, prec)).sum(), xa[1])[0]
+    assert float((got["tf32x3"] - got["fp64"]).norm()) <= 2.0 ** -22 * float(got["fp64"].norm())
